@@ -157,7 +157,8 @@ int ves3d_sv_launch_eval_graph(ves3d_sv* sv);
  * (precision, points, vesicles and their sizes) every candidate shape -- waves of CTAs
  * per SM in {4, 8, 16} x threads per CTA in {256, 384} (two targets each; the mixed form
  * 256 only, for its accuracy) -- is timed once with CUDA events and the fastest is kept.
- * Never tunes during stream capture. */
+ * FP64 sums over 8000 and more points have one form that needs no tuning (every unordered
+ * pair evaluated once) unless a shape is fixed. Never tunes during stream capture. */
 int ves3d_set_autotune(int on);
 /* Fix the far-field launch shape instead (waves in {4, 8, 16}, threads per CTA in
  * {256, 384}, targets per thread 2); waves = 0 returns to the default / autotuned shape. */

@@ -89,6 +89,12 @@ __device__ __forceinline__ double rsqrt_f64_int_seed(double r2) {
 // Coincidence test on the high word of a squared distance: true for r2 >= 2^-126.
 __device__ __forceinline__ bool r2_normal(double r2) { return __double2hiint(r2) >= 0x38100000; }
 
+// The same with squared distances of 2^128 and more (beyond the seed's range) cut off as well: such
+// a pair contributes nothing.
+__device__ __forceinline__ bool r2_in_range(double r2) {
+  return (unsigned)(__double2hiint(r2) - 0x38100000) < 0x0FE00000u;
+}
+
 __device__ __forceinline__ double rsqrt_f64(double r2) {
   double y = (double)rsqrtf((float)r2);
   double e = fma(-r2 * y, y, 1.0);

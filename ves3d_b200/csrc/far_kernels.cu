@@ -13,7 +13,8 @@
 // its segment; k_far_reduce adds the segments in a fixed order (the result is
 // deterministic) and fuses the addition of the self part.
 //
-// FP64 form: two independent FP64 chains per thread; 1/sqrt from an FP32 hardware seed
+// FP64 form (fewer points than kFarSymMin, or a forced launch shape; more take the paired sums of
+// far_sym_kernels.cu): two independent FP64 chains per thread; 1/sqrt from an FP32 hardware seed
 // refined in FP64; a coincident pair (|r| = 0) contributes nothing, as in the reference.
 // Mixed form: coordinates relative to the centroid of the chunk's targets (differences
 // taken in FP64, rounded to FP32 once per source per CTA), the pair arithmetic in packed
@@ -36,6 +37,10 @@
 namespace ves3d {
 
 constexpr int kTileF64 = 512;  // 24.6 KB staged per barrier pair (2% faster than 256 at 512 vesicles)
+// Small suspensions (below kFarSymMin points, the one-sided FP64 form's range): 64-thread CTAs and
+// segments of whole 32-source tiles, so that a few thousand points still make hundreds of CTAs
+// (2,496 points in 20 CTAs of 384 threads: 181 us; in 64-thread CTAs 19 us).
+constexpr int kTileSmall = 32, kThreadsSmall = 64;
 // FP32 form: 960 sources staged per pair of barriers (46 KB of shared memory), summed in
 // FP32 over sub-tiles of 120 and the sub-tile sums added in FP64. Measured against
 // 512-source tiles summed whole in FP32: 12% shorter launches at 512 vesicles, and the far
@@ -135,12 +140,12 @@ __device__ __forceinline__ void stage64(double* sm, const double* __restrict__ a
 // grid (segments, target chunks of 2 NT); pos/den point-major [N][3]; part [seg][N][3].
 // 384 threads at 56 registers: three CTAs (36 warps) per SM, measured 16% faster at 512
 // vesicles than one vesicle per CTA at 288 threads and 63 registers.
-template <int NT>
+template <int NT, int TILE>
 __global__ void __launch_bounds__(NT, 1152 / NT) k_far_f64_flat(const double* __restrict__ pos,
                                                                  const double* __restrict__ den,
                                                                  const long* __restrict__ off, long nves, long N,
                                                                  int seg_tiles, double* __restrict__ part) {
-  __shared__ __align__(16) double sm[kTileF64 * 6];
+  __shared__ __align__(16) double sm[TILE * 6];
   __shared__ ChunkRange cr;
   chunk_range<NT>(off, nves, N, &cr);
   const int seg = blockIdx.x;
@@ -150,11 +155,11 @@ __global__ void __launch_bounds__(NT, 1152 / NT) k_far_f64_flat(const double* __
   const double ax_ = pos[3 * la], ay_ = pos[3 * la + 1], az_ = pos[3 * la + 2];
   const double bx_ = pos[3 * lb], by_ = pos[3 * lb + 1], bz_ = pos[3 * lb + 2];
   Acc64 A, B;
-  const long ntiles = (N + kTileF64 - 1) / kTileF64;
+  const long ntiles = (N + TILE - 1) / TILE;
   const long tb = (long)seg * seg_tiles, te = min(tb + seg_tiles, ntiles);
   for (long tile = tb; tile < te; tile++) {
-    const long s0 = tile * kTileF64;
-    const int ns = (int)min((long)kTileF64, N - s0);
+    const long s0 = tile * TILE;
+    const int ns = (int)min((long)TILE, N - s0);
     __syncthreads();
     stage64<6, NT>(sm, pos, den, nullptr, s0, ns);
     __syncthreads();
@@ -172,12 +177,12 @@ __global__ void __launch_bounds__(NT, 1152 / NT) k_far_f64_flat(const double* __
     }
   }
   // the chunk's own vesicles within this segment: each target skips its own vesicle
-  const long g0 = max(cr.u0, tb * kTileF64), g1 = min(cr.u1, min(te * kTileF64, N));
+  const long g0 = max(cr.u0, tb * TILE), g1 = min(cr.u1, min(te * TILE, N));
   if (g0 < g1) {
     const long va = vesicle_of(off, nves, la), vb = vesicle_of(off, nves, lb);
     const long ea0 = off[va], ea1 = off[va + 1], eb0 = off[vb], eb1 = off[vb + 1];
-    for (long s0 = g0; s0 < g1; s0 += kTileF64) {
-      const int ns = (int)min((long)kTileF64, g1 - s0);
+    for (long s0 = g0; s0 < g1; s0 += TILE) {
+      const int ns = (int)min((long)TILE, g1 - s0);
       __syncthreads();
       stage64<6, NT>(sm, pos, den, nullptr, s0, ns);
       __syncthreads();
@@ -221,13 +226,13 @@ __device__ __forceinline__ void pair_dl64(const double* s, double tx, double ty,
   a.z = fma(dz, q, a.z);
 }
 
-template <int NT>
+template <int NT, int TILE>
 __global__ void __launch_bounds__(NT, 1152 / NT) k_far_dl_f64_flat(const double* __restrict__ pos,
                                                                     const double* __restrict__ nrm,
                                                                     const double* __restrict__ dden,
                                                                     const long* __restrict__ off, long nves, long N,
                                                                     int seg_tiles, double* __restrict__ part) {
-  __shared__ __align__(16) double sm[kTileF64 * 9];
+  __shared__ __align__(16) double sm[TILE * 9];
   __shared__ ChunkRange cr;
   chunk_range<NT>(off, nves, N, &cr);
   const int seg = blockIdx.x;
@@ -237,11 +242,11 @@ __global__ void __launch_bounds__(NT, 1152 / NT) k_far_dl_f64_flat(const double*
   const double ax_ = pos[3 * la], ay_ = pos[3 * la + 1], az_ = pos[3 * la + 2];
   const double bx_ = pos[3 * lb], by_ = pos[3 * lb + 1], bz_ = pos[3 * lb + 2];
   Acc64 A, B;
-  const long ntiles = (N + kTileF64 - 1) / kTileF64;
+  const long ntiles = (N + TILE - 1) / TILE;
   const long tb = (long)seg * seg_tiles, te = min(tb + seg_tiles, ntiles);
   for (long tile = tb; tile < te; tile++) {
-    const long s0 = tile * kTileF64;
-    const int ns = (int)min((long)kTileF64, N - s0);
+    const long s0 = tile * TILE;
+    const int ns = (int)min((long)TILE, N - s0);
     __syncthreads();
     stage64<9, NT>(sm, pos, nrm, dden, s0, ns);
     __syncthreads();
@@ -256,12 +261,12 @@ __global__ void __launch_bounds__(NT, 1152 / NT) k_far_dl_f64_flat(const double*
       pair_dl64(sm + 9 * k, bx_, by_, bz_, B);
     }
   }
-  const long g0 = max(cr.u0, tb * kTileF64), g1 = min(cr.u1, min(te * kTileF64, N));
+  const long g0 = max(cr.u0, tb * TILE), g1 = min(cr.u1, min(te * TILE, N));
   if (g0 < g1) {
     const long va = vesicle_of(off, nves, la), vb = vesicle_of(off, nves, lb);
     const long ea0 = off[va], ea1 = off[va + 1], eb0 = off[vb], eb1 = off[vb + 1];
-    for (long s0 = g0; s0 < g1; s0 += kTileF64) {
-      const int ns = (int)min((long)kTileF64, g1 - s0);
+    for (long s0 = g0; s0 < g1; s0 += TILE) {
+      const int ns = (int)min((long)TILE, g1 - s0);
       __syncthreads();
       stage64<9, NT>(sm, pos, nrm, dden, s0, ns);
       __syncthreads();
@@ -706,22 +711,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_far_dl_f32_flat(const double*
   }
 }
 
-// out (AxisMajor per vesicle) = add + (1/8pi) sum over segments in order. One CTA per
-// vesicle; vesicle v holds points [off[v], off[v+1]) as [3][n_v] from 3*off[v].
+// out (AxisMajor per vesicle) = add + (1/8pi) sum over segments in order. CTAs (vesicle, part of
+// its values); vesicle v holds points [off[v], off[v+1]) as [3][n_v] from 3*off[v].
 __global__ void k_far_reduce(const double* __restrict__ part, int nseg, const long* __restrict__ off, long N,
                              const double* __restrict__ add, double* __restrict__ out, double* __restrict__ far_out,
                              const double* __restrict__ part2, int nseg2, double scale2) {
   const int v = blockIdx.x;
   const long t0 = off[v], nt = off[v + 1] - t0;
-  for (long i = threadIdx.x; i < 3 * nt; i += blockDim.x) {
+  for (long i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * nt; i += (long)gridDim.y * blockDim.x) {
     const long k = i / 3;
     const int c = (int)(i - 3 * k);
     const long g = t0 + k;
     double s = 0.0;
+#pragma unroll 8
     for (int q = 0; q < nseg; q++) s += part[(long)q * 3 * N + 3 * g + c];
     s *= kInv8Pi;
     if (part2) {  // a second set of partials (the double layer) with its own constant
       double s2 = 0.0;
+#pragma unroll 8
       for (int q = 0; q < nseg2; q++) s2 += part2[(long)q * 3 * N + 3 * g + c];
       s += s2 * scale2;
     }
@@ -731,18 +738,23 @@ __global__ void k_far_reduce(const double* __restrict__ part, int nseg, const lo
   }
 }
 
+// 128-thread CTAs per vesicle: one round at p = 16 (1632 values). The kernel reads the partial sums
+// once; one CTA per vesicle left 64 vesicles on 64 SMs (69 us, now 26).
+constexpr int kReduceParts = 12;
+
 // Launch shape of the far field: how many waves of CTAs the source range is split into
 // (segments) and the threads of a CTA (two targets each).
 struct FarShape {
   int waves = 8;
   int nthr = 384;
+  int tile(bool mixed) const { return mixed ? kTileF32 : nthr == kThreadsSmall ? kTileSmall : kTileF64; }
 };
 
-// Default shapes, measured at 512 vesicles of p = 16 (one B200): FP64 16 waves of
-// 384-thread CTAs (122.5 ms); FP32 16 waves of 256-thread CTAs (384-thread chunks ran 46.3 ms
+// Default shapes: FP64 (small suspensions; larger ones take launch_far_sym) the small shape; FP32
+// 16 waves of 256-thread CTAs, measured at 512 vesicles of p = 16 (384-thread chunks ran 46.3 ms
 // with a larger worst-point error, 5.0e-7 against 3.2e-7: their origins lie farther from
 // some of their targets, so the FP32 form tunes over 256-thread CTAs only).
-static FarShape default_shape(bool mixed) { return mixed ? FarShape{16, 256} : FarShape{16, 384}; }
+static FarShape default_shape(bool mixed) { return mixed ? FarShape{16, 256} : FarShape{16, kThreadsSmall}; }
 
 static int num_sms() {
   int dev = 0, nsm = 148;
@@ -765,7 +777,8 @@ static int far_segments(long nchunk, long N, int tile, int nthr, int waves, long
 
 int launch_far_reduce(const double* part, int nseg, const long* off, long nves, long N, const double* add, double* out,
                       double* far_out, cudaStream_t st, const double* part2, int nseg2, double scale2) {
-  k_far_reduce<<<(unsigned)nves, 256, 0, st>>>(part, nseg, off, N, add, out, far_out, part2, nseg2, scale2);
+  k_far_reduce<<<dim3((unsigned)nves, kReduceParts), 128, 0, st>>>(part, nseg, off, N, add, out, far_out, part2, nseg2,
+                                                                   scale2);
   VES3D_LAUNCHED();
   return VES3D_OK;
 }
@@ -779,17 +792,19 @@ static int launch_far_shape(const FarShape& sh, bool mixed, const double* pos, c
     return VES3D_ERR_ARG;
   }
   int seg_tiles = 1;
-  const int nseg = far_segments(nchunk, N, mixed ? kTileF32 : kTileF64, sh.nthr, sh.waves, part_cap_segments,
-                                &seg_tiles);
+  const long cap = sh.nthr == kThreadsSmall ? part_cap_segments : std::min(part_cap_segments, kFarMaxSegments);
+  const int nseg = far_segments(nchunk, N, sh.tile(mixed), sh.nthr, sh.waves, cap, &seg_tiles);
   dim3 grid((unsigned)nseg, (unsigned)nchunk);
   if (mixed && sh.nthr == 384)
     k_far_f32_flat<384><<<grid, 384, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
   else if (mixed)
     k_far_f32_flat<256><<<grid, 256, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
+  else if (sh.nthr == kThreadsSmall)
+    k_far_f64_flat<kThreadsSmall, kTileSmall><<<grid, kThreadsSmall, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
   else if (sh.nthr == 384)
-    k_far_f64_flat<384><<<grid, 384, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
+    k_far_f64_flat<384, kTileF64><<<grid, 384, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
   else
-    k_far_f64_flat<256><<<grid, 256, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
+    k_far_f64_flat<256, kTileF64><<<grid, 256, 0, st>>>(pos, den, off, nves, N, seg_tiles, part);
   VES3D_LAUNCHED();
   *nseg_out = nseg;
   return VES3D_OK;
@@ -903,10 +918,18 @@ int launch_far_groups(bool mixed, const double* pos, const double* den, const lo
     if (nseg_out) *nseg_out = 0;
     return VES3D_OK;
   }
+  int s, nseg = 0;
+  if (!mixed && N >= kFarSymMin && !g_forced.waves) {
+    if ((s = launch_far_sym(pos, den, nullptr, off, nves, N, part, part_cap_segments, st, &nseg))) return s;
+    if (nseg_out) {
+      *nseg_out = nseg;
+      return VES3D_OK;
+    }
+    return launch_far_reduce(part, nseg, off, nves, N, add, out, far_out, st);
+  }
   FarShape shape;
-  int s = tuned_shape(mixed, pos, den, off, nves, N, groups, ngroups, part, part_cap_segments, st, &shape);
+  s = tuned_shape(mixed, pos, den, off, nves, N, groups, ngroups, part, part_cap_segments, st, &shape);
   if (s) return s;
-  int nseg = 0;
   if ((s = launch_far_shape(shape, mixed, pos, den, off, nves, N, part, part_cap_segments, st, &nseg))) return s;
   if (nseg_out) {
     *nseg_out = nseg;
@@ -947,23 +970,20 @@ int launch_far_dl_groups(bool mixed, const double* pos, const double* nrm, const
       return VES3D_ERR_ARG;
     }
     int seg_tiles = 1;
-    const int nseg = far_segments(nchunk, N, kTileDL32, NT, 16, part_cap_segments, &seg_tiles);
+    const int nseg = far_segments(nchunk, N, kTileDL32, NT, 16, std::min(part_cap_segments, kFarMaxSegments), &seg_tiles);
     k_far_dl_f32_flat<NT><<<dim3((unsigned)nseg, (unsigned)nchunk), NT, 0, st>>>(pos, nrm, dden, off, nves, N,
                                                                                  seg_tiles, part);
     VES3D_LAUNCHED();
     *nseg_out = nseg;
     return VES3D_OK;
   }
-  constexpr int NT = 384;
+  if (N >= kFarSymMin) return launch_far_sym(pos, dden, nrm, off, nves, N, part, part_cap_segments, st, nseg_out);
+  constexpr int NT = kThreadsSmall;
   const long nchunk = (N + 2L * NT - 1) / (2L * NT);
-  if (nchunk > 65535) {
-    set_error("far double layer: %ld points exceed the launch's %ld target chunks", N, 65535L * 2 * NT);
-    return VES3D_ERR_ARG;
-  }
   int seg_tiles = 1;
-  const int nseg = far_segments(nchunk, N, kTileF64, NT, 8, part_cap_segments, &seg_tiles);
-  k_far_dl_f64_flat<NT><<<dim3((unsigned)nseg, (unsigned)nchunk), NT, 0, st>>>(pos, nrm, dden, off, nves, N,
-                                                                               seg_tiles, part);
+  const int nseg = far_segments(nchunk, N, kTileSmall, NT, 16, part_cap_segments, &seg_tiles);
+  k_far_dl_f64_flat<NT, kTileSmall><<<dim3((unsigned)nseg, (unsigned)nchunk), NT, 0, st>>>(pos, nrm, dden, off, nves, N,
+                                                                                           seg_tiles, part);
   VES3D_LAUNCHED();
   *nseg_out = nseg;
   return VES3D_OK;

@@ -150,6 +150,18 @@ int launch_direct_stokes_dl_f64(int src_m, int trg_m, int n, int t_head, int t_t
                                 const double* S, const double* N, const double* D, double* U, const double* Q,
                                 cudaStream_t st);
 constexpr long kFarMaxSegments = 32;
+// From this many points on, the FP64 far field evaluates each unordered pair once
+// (far_sym_kernels.cu); fewer make too few items of it to fill the chip. One-sided and paired, us:
+// 6,528 points 91 and 98 (double layer 106 and 107), 7,616 points 115 and 125 (133 and 129), 8,704
+// points 151 and 134 (176 and 149).
+constexpr long kFarSymMin = 8000;
+// Sets of partial sums a far field of N points is given room for.
+long far_slots(long N);
+// All unordered pairs of points of different vesicles (off null: all pairs), FP64: the single
+// layer of den, or with nrm the double layer (unscaled, as the partials of launch_far and
+// launch_far_dl); part [*nslots][N][3], *nslots <= max_slots.
+int launch_far_sym(const double* pos, const double* den, const double* nrm, const long* off, long nves, long N,
+                   double* part, long max_slots, cudaStream_t st, int* nslots);
 // Vesicles [v0, v0 + nv) all with nt points: one far-field launch each, sized for nt.
 struct FarGroup {
   long v0, nv;

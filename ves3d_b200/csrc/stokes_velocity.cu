@@ -312,6 +312,11 @@ struct ves3d_sv {
     chunk = 0;
   }
   long npts() const { return nves * ngrid_(p); }
+  // sets of far-field partial sums of the current points that the buffers (sized for cap_ves) hold
+  long part_slots() const {
+    const long cap = cap_ves * ngrid_(p);
+    return far_slots(cap) * cap / npts();
+  }
 };
 
 namespace {
@@ -344,7 +349,6 @@ int alloc_resident(ves3d_sv* sv, long nves) {
   s |= dalloc(&sv->SL, (size_t)nves * n * n);
   s |= dalloc(&sv->Fc, (size_t)nves * n);
   s |= dalloc(&sv->Vc, (size_t)nves * n);
-  s |= dalloc(&sv->part, (size_t)kFarMaxSegments * fld);
   s |= dalloc(&sv->off, (size_t)nves + 1);
   if (s) {
     sv->free_buffers();
@@ -366,7 +370,7 @@ int alloc_dl(ves3d_sv* sv) {
   s |= dalloc(&sv->DL, (size_t)nves * n * n);
   s |= dalloc(&sv->nrm, fld);
   s |= dalloc(&sv->dden, fld);
-  s |= dalloc(&sv->part_dl, (size_t)kFarMaxSegments * fld);
+  s |= dalloc(&sv->part_dl, (size_t)far_slots(nves * ng) * fld);
   if (s) {
     sv->free_dl();
     return s;
@@ -599,12 +603,16 @@ int fork_far(ves3d_sv* sv, int* nseg, cudaEvent_t ev_far0, cudaEvent_t ev_far1, 
   const DevTables& T = sv->tab->d;
   int s;
   cudaStream_t fs = sv->overlap ? sv->side : sv->stream;
+  if (!sv->part) {  // (an order group of a polydisperse suspension never comes here)
+    const long cap = sv->cap_ves * ngrid_(sv->p);
+    if ((s = dalloc(&sv->part, (size_t)far_slots(cap) * 3 * cap))) return s;
+  }
   VES3D_CK(cudaEventRecord(sv->ev_fork, sv->stream));
   VES3D_CK(cudaStreamWaitEvent(fs, sv->ev_fork, 0));
   if ((s = launch_far_density(sv->F, sv->area, sv->nves, sv->p, T.smooth_w0, sv->den, fs))) return s;
   if (ev_far0) VES3D_CK(cudaEventRecord(ev_far0, fs));
   if ((s = launch_far(sv->prec == VES3D_PREC_MIXED && !sv->far_force_fp64, sv->pos, sv->den, sv->off, sv->nves,
-                      sv->npts(), ngrid_(sv->p), nullptr, nullptr, nullptr, sv->part, kFarMaxSegments, fs, nseg)))
+                      sv->npts(), ngrid_(sv->p), nullptr, nullptr, nullptr, sv->part, sv->part_slots(), fs, nseg)))
     return s;
   if (ev_far1) VES3D_CK(cudaEventRecord(ev_far1, fs));
   sv->nseg_dl = 0;
@@ -614,7 +622,7 @@ int fork_far(ves3d_sv* sv, int* nseg, cudaEvent_t ev_far0, cudaEvent_t ev_far1, 
     if (ev_far0) VES3D_CK(cudaEventRecord(sv->ev[8], fs));
     const bool dl32 = sv->prec == VES3D_PREC_MIXED && !sv->far_force_fp64 && sv->far_dl_f32;
     if ((s = launch_far_dl(dl32, sv->pos, sv->nrm, sv->dden, sv->off, sv->nves, sv->npts(), ngrid_(sv->p),
-                           sv->part_dl, kFarMaxSegments, fs, &sv->nseg_dl)))
+                           sv->part_dl, sv->part_slots(), fs, &sv->nseg_dl)))
       return s;
     if (ev_far0) VES3D_CK(cudaEventRecord(sv->ev[9], fs));
   }
@@ -3052,6 +3060,8 @@ struct ves3d_svp {
     graph_exec = nullptr;
     graph = nullptr;
   }
+  // sets of far-field partial sums of the current points that the buffers (sized for capN) hold
+  long part_slots() const { return far_slots(capN) * capN / N; }
   void free_global() {
     double* ps[] = {pos, den, vself, V, Vfar, part, nrm, dden, part_dl};
     for (double* q : ps) dfree(q);
@@ -3167,7 +3177,7 @@ int ves3d_svp_set_src_coord(ves3d_svp* g, const double* S, const int* orders, lo
     s |= dalloc(&g->vself, 3 * (size_t)pt);
     s |= dalloc(&g->V, 3 * (size_t)pt);
     s |= dalloc(&g->Vfar, 3 * (size_t)pt);
-    s |= dalloc(&g->part, (size_t)kFarMaxSegments * 3 * pt);
+    s |= dalloc(&g->part, (size_t)far_slots(pt) * 3 * pt);
     s |= dalloc(&g->off, (size_t)n_ves + 1);
     if (s) {
       g->free_global();
@@ -3209,7 +3219,7 @@ static int svp_alloc_dl(ves3d_svp* g) {
   if (g->nrm) return VES3D_OK;
   s |= dalloc(&g->nrm, 3 * (size_t)g->capN);
   s |= dalloc(&g->dden, 3 * (size_t)g->capN);
-  s |= dalloc(&g->part_dl, (size_t)kFarMaxSegments * 3 * g->capN);
+  s |= dalloc(&g->part_dl, (size_t)far_slots(g->capN) * 3 * g->capN);
   if (s) {
     dfree(g->nrm);
     dfree(g->dden);
@@ -3293,13 +3303,13 @@ static int svp_far(ves3d_svp* g, bool dl) {
   }
   if (!dl)
     return launch_far_groups(mixed, g->pos, g->den, g->off, g->nves, g->N, fg.data(), (int)fg.size(), g->vself, g->V,
-                             g->Vfar, g->part, kFarMaxSegments, g->stream);
+                             g->Vfar, g->part, g->part_slots(), g->stream);
   int s, nseg = 0, nseg_dl = 0;
   if ((s = launch_far_groups(mixed, g->pos, g->den, g->off, g->nves, g->N, fg.data(), (int)fg.size(), nullptr,
-                             nullptr, nullptr, g->part, kFarMaxSegments, g->stream, &nseg)))
+                             nullptr, nullptr, g->part, g->part_slots(), g->stream, &nseg)))
     return s;
   if ((s = launch_far_dl_groups(mixed && g->far_dl_f32, g->pos, g->nrm, g->dden, g->off, g->nves, g->N, fg.data(),
-                                (int)fg.size(), g->part_dl, kFarMaxSegments, g->stream, &nseg_dl)))
+                                (int)fg.size(), g->part_dl, g->part_slots(), g->stream, &nseg_dl)))
     return s;
   return launch_far_reduce(g->part, nseg, g->off, g->nves, g->N, g->vself, g->V, g->Vfar, g->stream, g->part_dl,
                            nseg_dl, kDl);
