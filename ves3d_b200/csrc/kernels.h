@@ -2,6 +2,7 @@
 #pragma once
 
 #include <string>
+#include <vector>
 #include <cuda_runtime.h>
 
 namespace ves3d {
@@ -25,6 +26,11 @@ struct DevTables {
   double *syn0_d2leg = nullptr, *syn0_d2four = nullptr;
   // syn1_leg / syn1_dleg transposed to [latitude][coefficient] (contiguous per latitude)
   double *syn1_leg_t = nullptr, *syn1_dleg_t = nullptr;
+  // the fused build's: the same times sqrt(2 pi) in rows of ring_ldl with blocks starting at ring_off
+  // (ring_leg_offsets); cos and sin of m phi_j, [p1 / 2 + 1][padded order + 1][2]
+  double *ring_leg = nullptr, *ring_dleg = nullptr, *ring_twiddle = nullptr;
+  int* ring_off = nullptr;
+  int ring_ldl = 0;
 };
 
 // Geometry record per point: E, F, G (divided by W^2), W, n[3], cu[3], cv[3], H, K.
@@ -90,10 +96,14 @@ int launch_rotate_transpose_f32(const float* C, long nv, const DevTables& T, flo
 // instantiated for (the mixed form's self matrices at p = 12 and 24).
 bool rotate_transpose_f32_from_f64_supported(int p0);
 int launch_rotate_transpose_f32(const double* C, long nv, const DevTables& T, float* SL3, cudaStream_t st);
-// Fused per-rotation build (FP64 tensor cores): R [nrot][3][Nc] -> C [nrot][2][6][Nc],
-// i.e. upsampled synthesis + singular kernel + transposed synthesis in one kernel.
-bool fused_build_supported(int p0, int p1);
-int launch_build_ring(const double* R, long nrot, const DevTables& T, double* C, cudaStream_t st);
+// Fused per-rotation build: R [nrot][3][Nc] -> C [nrot][2][6][Nc], i.e. upsampled synthesis +
+// singular kernel + transposed synthesis in one kernel.
+// For the single or the double layer (dl), any 2 <= p0 <= 24 and p0 <= p1 <= 56.
+bool ring_supported(int p0, int p1);
+// The order that the tables of the run-time instance taking (p0, p1) are padded to; 0: none needed.
+int ring_padded_order(int p0, int p1);
+std::vector<int> ring_leg_offsets(int p0);
+int launch_ring_build(bool dl, const double* R, long nrot, const DevTables& T, double* C, cudaStream_t st);
 // Mixed form of the fused build: the DFT GEMMs on tcgen05 tensor cores as split-BF16
 // products with FP32 accumulation (Legendre sums, kernel and targets FP64); same layouts.
 bool tc_build_supported(int p0, int p1);

@@ -7,6 +7,7 @@
 //                  -> singular kernel -> SHC2GridTranspose(p_up -> p) -> RotateTranspose
 //                  + Rearrange -> Grid2SHC -> SL [v][3Nc][3Nc]
 //                  (SphericalHarmonics::StokesSingularInteg_, src/SphericalHarmonics.cc:954-1180)
+//                  (the stages from SHC2Grid to its transpose are one kernel, ring_kernels.cu)
 //   eval         : Fc = Grid2SHC(f); Vc = Fc . SL; Vself = SHC2Grid(Vc)
 //                  (src/StokesVelocity.cc:385-473); den = f * area * qw;
 //                  vel = Vself + sum over other vesicles (exact all-pairs far field).
@@ -70,7 +71,7 @@ struct TablesOwner {
                     d.syn1_dleg, d.syn1_four, d.syn1_dfour, d.synT_four, d.jf_of_coef, d.blk_off, d.m_of_coef,
                     d.n_of_coef, d.partner, d.is_sin, d.mr, d.mr_off, d.perm, d.perm_off, d.pos_in_block,
                     d.sing_w, d.smooth_w0, d.qp, d.cos_tab, d.sin_tab, d.syn0_d2leg, d.syn0_d2four,
-                    d.syn1_leg_t, d.syn1_dleg_t};
+                    d.syn1_leg_t, d.syn1_dleg_t, d.ring_leg, d.ring_dleg, d.ring_twiddle, d.ring_off};
     for (void* p : ptrs) dfree(p);
   }
   int upload(cudaStream_t st) {
@@ -98,8 +99,34 @@ struct TablesOwner {
           }
         s |= dupload(&d.syn1_leg_t, a, st);
         s |= dupload(&d.syn1_dleg_t, b, st);
+        const std::vector<int> lo = ring_leg_offsets(h.p0);
+        const size_t ldl = lo.back();
+        const double scale = std::sqrt(2.0 * M_PI);
+        std::vector<double> ra(ldl * nl, 0.0), rb(ldl * nl, 0.0);
+        for (size_t l = 0; l < nl; l++)
+          for (int k = 0; k < 2 * h.p0; k++) {
+            const int b0 = h.blk_off[k], len = h.blk_off[k + 1] - b0;
+            for (int i = 0; i < len; i++) {  // even degrees of the block first
+              const size_t o = l * ldl + lo[2 * k + i % 2] + i / 2;
+              ra[o] = a[l * nc + b0 + i] * scale;
+              rb[o] = b[l * nc + b0 + i] * scale;
+            }
+          }
+        d.ring_ldl = (int)ldl;
+        s |= dupload(&d.ring_off, lo, st);
+        s |= dupload(&d.ring_leg, ra, st);
+        s |= dupload(&d.ring_dleg, rb, st);
       }
     }
+    const int pad = ring_supported(h.p0, h.p1) ? ring_padded_order(h.p0, h.p1) : 0;
+    std::vector<double> tw;
+    for (int j = 0; pad && j <= h.p1 / 2; j++)
+      for (int m = 0; m <= pad; m++) {
+        const double a = M_PI * ((long)m * j % (2 * h.p1)) / h.p1;
+        tw.push_back(std::cos(a));
+        tw.push_back(std::sin(a));
+      }
+    s |= dupload(&d.ring_twiddle, tw, st);
     s |= dupload(&d.syn1_four, h.syn1.four, st);
     s |= dupload(&d.syn1_dfour, h.syn1.dfour, st);
     s |= dupload(&d.synT_four, h.synT.four, st);
@@ -384,7 +411,7 @@ int alloc_dl(ves3d_sv* sv) {
 bool use_fused(const ves3d_sv* sv) {
   const char* env = getenv("VES3D_FUSED_BUILD");
   if (env && env[0] == '0') return false;
-  return fused_build_supported(sv->p, sv->pup);
+  return ring_supported(sv->p, sv->pup);
 }
 
 // The mixed form builds with the DFT GEMMs on tcgen05 tensor cores where that kernel is
@@ -483,8 +510,7 @@ int copy_out(double* dst, const double* src, size_t n, int is_device, cudaStream
 int alloc_scratch(ves3d_sv* sv);
 int run_setup(ves3d_sv* sv, bool dl = false);
 
-// The self matrices of every vesicle: the single layer (SL), or with dl the double layer
-// (DL, always by the stage-by-stage pipeline).
+// The self matrices of every vesicle: the single layer (SL), or with dl the double layer (DL).
 int run_setup(ves3d_sv* sv, bool dl) {
   NvtxRange nvtx(dl ? "ves3d build dl" : "ves3d build");
   const DevTables& T = sv->tab->d;
@@ -493,9 +519,9 @@ int run_setup(ves3d_sv* sv, bool dl) {
   cudaStream_t st = sv->stream;
   int s = alloc_scratch(sv);
   if (s) return s;
-  const bool fused = !dl && use_fused(sv);
-  const bool tc = fused && use_tc_build(sv);
-  const bool f32post = fused && !tc && use_f32_post(sv);
+  const bool fused = use_fused(sv);
+  const bool tc = !dl && fused && use_tc_build(sv);
+  const bool f32post = !dl && fused && !tc && use_f32_post(sv);
   double* M = dl ? sv->DL : sv->SL;
   if ((!fused && !sv->K) || !M) {
     set_error("internal: self-matrix build without its buffers");
@@ -512,7 +538,7 @@ int run_setup(ves3d_sv* sv, bool dl) {
     if (fused && tc) {
       if ((s = launch_build_ring_tc(sv->R, nrot, T, Cf, st))) return s;
     } else if (fused) {
-      if ((s = launch_build_ring(sv->R, nrot, T, sv->C, st))) return s;
+      if ((s = launch_ring_build(dl, sv->R, nrot, T, sv->C, st))) return s;
     } else {
       if ((s = launch_synthesis(sv->R, nrot * 3, p0, p1, T.syn1_leg, T.syn1_dleg, T.syn1_four, T.syn1_dfour,
                                 T.blk_off, sv->Xu, sv->Xut, sv->Xup, st)))
