@@ -150,7 +150,8 @@ int launch_far_dl(bool mixed, const double* pos, const double* nrm, const double
 // layer of den, plus with nrm non-null the double layer of nrm and dden (all point-major,
 // densities times area and weights).
 int launch_targets_f64(const double* pos, const double* den, const double* nrm, const double* dden, long N,
-                       const double* trg, long M, double* out, cudaStream_t st);
+                       const double* trg, long M, double* out, double* part, cudaStream_t st);
+size_t targets_part_doubles(long M);  // of part, the partial sums of few targets' source segments
 // Unit outward normals (X_theta x X_phi) / |X_theta x X_phi| of nv surfaces at order p0,
 // AxisMajor derivatives in, point-major [N][3] out.
 int launch_unit_normals(const double* Xt, const double* Xp, long nv, int p0, double* nrm, cudaStream_t st);
@@ -191,8 +192,13 @@ int launch_far_dl_groups(bool mixed, const double* pos, const double* nrm, const
                          cudaStream_t st, int* nseg_out);
 // out = a + b elementwise.
 int launch_add(const double* a, const double* b, long n, double* out, cudaStream_t st);
-// All pairs, point-major in/out (StokesAlltoAll semantics).
-int launch_alltoall_f64(const double* pos, const double* den, long np, double* pot, cudaStream_t st);
+// All pairs, point-major in/out (StokesAlltoAll semantics). With part ([slots][np][3]) each
+// unordered pair is evaluated once (launch_far_sym); without, nothing but the arguments is used.
+int launch_alltoall_f64(const double* pos, const double* den, long np, double* pot, double* part, long slots,
+                        cudaStream_t st);
+// Slots worth giving it for np points: 0 where the one-sided form is the faster or the partial
+// sums would pass a GiB.
+long alltoall_slots(long np);
 // Per-surface DirectStokes with weights (cuda_stokes semantics).
 int launch_direct_stokes_f64(int src_m, int trg_m, int n, int t_head, int t_tail, const double* T,
                              const double* S, const double* D, double* U, const double* Q, cudaStream_t st);

@@ -69,7 +69,7 @@ int noalloc_body(const double* src, const double* den, size_t np, double* pot, c
   double* dpot = base + (size_t)6 * VES3D_NOALLOC_MAX_POINTS;
   VES3D_CK(cudaMemcpyAsync(dsrc, src, 3 * np * sizeof(double), cudaMemcpyHostToDevice, st));
   VES3D_CK(cudaMemcpyAsync(dden, den, 3 * np * sizeof(double), cudaMemcpyHostToDevice, st));
-  if ((s = launch_alltoall_f64(dsrc, dden, (long)np, dpot, st))) return s;
+  if ((s = launch_alltoall_f64(dsrc, dden, (long)np, dpot, nullptr, 0, st))) return s;
   VES3D_CK(cudaMemcpyAsync(pot, dpot, 3 * np * sizeof(double), cudaMemcpyDeviceToHost, st));
   VES3D_CK(cudaStreamSynchronize(st));
   return VES3D_OK;

@@ -193,7 +193,7 @@ struct ves3d_sv {
   std::vector<double> lam;
   bool contrast = false;
   // off-surface targets (SetTrgCoord): point-major [trg_n][3] and their velocities
-  double *trg = nullptr, *vtrg = nullptr;
+  double *trg = nullptr, *vtrg = nullptr, *trg_part = nullptr;  // (trg_part: partial sums)
   long trg_n = 0, trg_cap = 0;
   // near-singular correction of the targets (NearSingular): the upsampled sources of every
   // vesicle (surface, tangents, density, double-layer density at p_up, AxisMajor; area;
@@ -278,6 +278,7 @@ struct ves3d_sv {
     dfree(dlc);
     dfree(trg);
     dfree(vtrg);
+    dfree(trg_part);
     drop_graph();
     free_precond();
     for (auto& e : pc_ev)
@@ -811,7 +812,7 @@ int eval_trg_near(ves3d_sv* sv) {
   }
   // the smooth quadrature of every vesicle at every target
   if ((s = launch_targets_f64(sv->nu_pos, sv->nu_den, dl ? sv->nu_nrm : nullptr, dl ? sv->nu_dden : nullptr,
-                              nv * ng1, sv->trg, M, sv->vtrg, st)))
+                              nv * ng1, sv->trg, M, sv->vtrg, sv->trg_part, st)))
     return s;
   // r_near = r_ves 2 / sqrt(p_up) (src/NearSingular.cc:160, :119-158)
   if ((s = launch_centroid_radius(sv->X, nv, p, sv->nu_cen, sv->nu_rmax, st))) return s;
@@ -1021,9 +1022,12 @@ int ves3d_sv_set_trg_coord(ves3d_sv* sv, const double* T, long n_trg, int is_dev
   if (n_trg > sv->trg_cap) {
     dfree(sv->trg);
     dfree(sv->vtrg);
-    sv->trg = sv->vtrg = nullptr;
+    dfree(sv->trg_part);
+    sv->trg = sv->vtrg = sv->trg_part = nullptr;
     sv->trg_cap = 0;
-    if ((s = dalloc(&sv->trg, 3 * (size_t)n_trg)) || (s = dalloc(&sv->vtrg, 3 * (size_t)n_trg))) return s;
+    if ((s = dalloc(&sv->trg, 3 * (size_t)n_trg)) || (s = dalloc(&sv->vtrg, 3 * (size_t)n_trg)) ||
+        (s = dalloc(&sv->trg_part, targets_part_doubles(n_trg))))
+      return s;
     sv->trg_cap = n_trg;
   }
   if ((s = copy_in(sv->trg, T, 3 * (size_t)n_trg, is_device, sv->stream))) return s;
@@ -1052,7 +1056,8 @@ int ves3d_sv_eval_trg(ves3d_sv* sv, double* vel, int is_device) {
   }
   if (sv->near_on) {
     if ((s = eval_trg_near(sv))) return s;
-  } else if ((s = launch_targets_f64(sv->pos, sv->den, nrm, dden, sv->npts(), sv->trg, sv->trg_n, sv->vtrg, st))) {
+  } else if ((s = launch_targets_f64(sv->pos, sv->den, nrm, dden, sv->npts(), sv->trg, sv->trg_n, sv->vtrg,
+                                     sv->trg_part, st))) {
     return s;
   }
   return copy_out(vel, sv->vtrg, 3 * (size_t)sv->trg_n, is_device, st);
@@ -1575,11 +1580,11 @@ int ves3d_cuda_stokes_double_layer_f64(int src_m, int trg_m, int n, int t_head, 
 
 int ves3d_stokes_alltoall_device_f64(const double* src, const double* den, size_t np, double* pot, void* stream) {
   VES3D_ARG(src && den && pot, "null pointer");
-  return launch_alltoall_f64(src, den, (long)np, pot, (cudaStream_t)stream);
+  return launch_alltoall_f64(src, den, (long)np, pot, nullptr, 0, (cudaStream_t)stream);
 }
 
 struct InteractionWorkspace {
-  double* buf = nullptr;
+  double* buf = nullptr;  // sources, densities, potentials, then the partial sums of the paired form
   size_t cap = 0;
   cudaStream_t st = nullptr;
 };
@@ -1600,7 +1605,8 @@ void ves3d_stokes_alltoall_f64(const double* src, const double* den, size_t np, 
     if (!*ctx) *ctx = new InteractionWorkspace();
     ws = (InteractionWorkspace*)*ctx;
   }
-  const size_t need = 9 * np;
+  const long slots = alltoall_slots((long)np);
+  const size_t need = (9 + 3 * (size_t)slots) * np;
   if (ws->cap < need) {
     if (ws->buf) cudaFree(ws->buf);
     ws->buf = nullptr;
@@ -1622,7 +1628,7 @@ void ves3d_stokes_alltoall_f64(const double* src, const double* den, size_t np, 
   if (cudaMemcpyAsync(dsrc, src, 3 * np * sizeof(double), cudaMemcpyHostToDevice, ws->st) != cudaSuccess ||
       cudaMemcpyAsync(dden, den, 3 * np * sizeof(double), cudaMemcpyHostToDevice, ws->st) != cudaSuccess)
     s = VES3D_ERR_CUDA;
-  if (!s) s = launch_alltoall_f64(dsrc, dden, (long)np, dpot, ws->st);
+  if (!s) s = launch_alltoall_f64(dsrc, dden, (long)np, dpot, slots ? dpot + 3 * np : nullptr, slots, ws->st);
   if (!s && cudaMemcpyAsync(pot, dpot, 3 * np * sizeof(double), cudaMemcpyDeviceToHost, ws->st) != cudaSuccess)
     s = VES3D_ERR_CUDA;
   if (cudaStreamSynchronize(ws->st) != cudaSuccess) s = VES3D_ERR_CUDA;
