@@ -18,10 +18,13 @@
 // 3 x 3 grid points; here a target's near vesicles come from a bounding-sphere test and
 // its distance to the vesicle's upsampled points (up to kNearMax per target, ascending
 // vesicle order), and the projection is Gauss-Newton on the spherical-harmonic surface
-// itself from the nearest upsampled point: one warp per (target, vesicle) pair, lane m
-// carrying the order-m Legendre recurrence. The on-surface velocity and density at P come
+// itself from the nearest upsampled point: a warp or half a warp per (target, vesicle) pair, lane
+// m carrying the order-m Legendre recurrence. The on-surface velocity and density at P come
 // from their coefficients the same way. Each pair's correction is written to its own slot
 // and the slots are added in order (deterministic).
+#include <cmath>
+#include <vector>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -31,6 +34,7 @@ namespace {
 
 constexpr int kInterpDeg = 8;
 constexpr double kSqrt2Pi = 2.5066282746310002;
+constexpr double kStepDone = 1e-14;  // a Gauss-Newton step (radians) of no effect on the values
 
 __device__ __forceinline__ double inter_point(int i) { return i ? 1.0 + (i - 1.0) / (kInterpDeg - 2) : 0.0; }
 
@@ -82,124 +86,153 @@ __global__ void k_centroid_radius(const double* __restrict__ X, int ng, double* 
   }
 }
 
-// Near vesicles of each target: up to kNearMax in ascending vesicle order, with the index
-// of the nearest upsampled point; count[t] = their number, or kNearMax + 1 when more.
-__global__ void k_near_find(const double* __restrict__ trg, long M, const double* __restrict__ cen_r, long nv,
-                            const double* __restrict__ pos_up, int ng1, double r_near, int* __restrict__ count,
-                            int* __restrict__ near_v, int* __restrict__ near_k) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M) return;
-  const double tx = trg[3 * t], ty = trg[3 * t + 1], tz = trg[3 * t + 2];
-  const double rn2 = r_near * r_near;
-  int cnt = 0;
-  for (long v = 0; v < nv; v++) {
-    const double dx = tx - cen_r[4 * v], dy = ty - cen_r[4 * v + 1], dz = tz - cen_r[4 * v + 2];
-    // upsampled points lie within about R of the centroid; a generous bound
-    const double reach = 1.25 * cen_r[4 * v + 3] + r_near;
-    if (dx * dx + dy * dy + dz * dz > reach * reach) continue;
-    const double* P = pos_up + 3 * v * (long)ng1;
-    double best = rn2;
-    int kb = -1;
-    for (int k = 0; k < ng1; k++) {
-      const double ex = P[3 * k] - tx, ey = P[3 * k + 1] - ty, ez = P[3 * k + 2] - tz;
-      const double d2 = ex * ex + ey * ey + ez * ez;
-      if (d2 < best) {
-        best = d2;
-        kb = k;
-      }
-    }
-    if (kb < 0) continue;
-    if (cnt < kNearMax) {
-      near_v[t * kNearMax + cnt] = (int)v;
-      near_k[t * kNearMax + cnt] = kb;
-    }
-    cnt++;
-  }
-  count[t] = cnt <= kNearMax ? cnt : kNearMax + 1;
+// r_near = r_ves 2 / sqrt(p_up), r_ves from the bits of the largest vesicle radius
+__device__ __forceinline__ double near_radius(const unsigned long long* rmax_bits, int p_up) {
+  return __longlong_as_double((long long)rmax_bits[0]) * 2.0 / sqrt((double)p_up);
 }
 
-// Sums over lane m of the order-m blocks of the coefficients: value, d/dtheta, d/dphi of
-// the 3 functions S[3][nc] at (x = cos theta, phi), reduced over the warp (all lanes get
-// them). Lane m < p + 1 runs the normalised associated Legendre recurrence of order m
-// (the reference's LegPoly / LegPolyDeriv, src/SphericalHarmonics.cc:889-950; P(m + 1, n)
-// for the derivative comes from lane m + 1).
-__device__ void sh_point(const double* __restrict__ S, int p, const int* __restrict__ blk_off, double x, double phi,
-                         bool grads, double* val) {
+// Near vesicles of each target: up to kNearMax in ascending vesicle order, with the index
+// of the nearest upsampled point; count[t] = their number, or kNearMax + 1 when more (the first
+// such target goes to *over). One warp per target: its lanes test 32 vesicles' spheres at a time
+// and share the points of those in reach (a thread per target left 27 vesicles' tests and 1,200
+// points per near vesicle to one lane: 1.34 ms for 20,000 targets, now 44 us).
+__global__ void __launch_bounds__(128) k_near_find(const double* __restrict__ trg, long M,
+                                                   const double* __restrict__ cen_r, long nv,
+                                                   const double* __restrict__ pos_up, int p_up,
+                                                   const unsigned long long* __restrict__ rmax_bits,
+                                                   unsigned long long* __restrict__ over, int* __restrict__ count,
+                                                   int* __restrict__ near_v, int* __restrict__ near_k) {
   const int lane = threadIdx.x & 31;
-  const int m = lane;
-  const int nc = p * (p + 2);
-  const double s = sqrt(fmax(1.0 - x * x, 0.0));
-  double acc[9];
-#pragma unroll
-  for (int i = 0; i < 9; i++) acc[i] = 0.0;
-  // diagonal P(m, m)
-  double pmm = 0.28209479177387814;  // 1/sqrt(4 pi)
-  for (int i = 1; i <= m && i <= p; i++) pmm = -pmm * s * sqrt((2.0 * i + 1.0) / (2.0 * i));
-  double cm = 1.0, sm = 0.0, dcm = 0.0, dsm = 0.0;
-  if (m <= p) {
-    sincos(m * phi, &sm, &cm);
-    dcm = -m * sm;
-    dsm = m * cm;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= M) return;
+  const int ng1 = 2 * p_up * (p_up + 1);
+  const double r_near = near_radius(rmax_bits, p_up);
+  const double tx = trg[3 * t], ty = trg[3 * t + 1], tz = trg[3 * t + 2];
+  int cnt = 0;
+  for (long v0 = 0; v0 < nv; v0 += 32) {
+    bool reach = false;
+    if (v0 + lane < nv) {
+      const double* c = cen_r + 4 * (v0 + lane);
+      const double dx = tx - c[0], dy = ty - c[1], dz = tz - c[2];
+      // upsampled points lie within about R of the centroid; a generous bound
+      const double r = 1.25 * c[3] + r_near;
+      reach = !(dx * dx + dy * dy + dz * dz > r * r);
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, reach); todo; todo &= todo - 1) {
+      const long v = v0 + __ffs(todo) - 1;
+      const double* P = pos_up + 3 * v * (long)ng1;
+      double best = r_near * r_near;
+      int kb = ng1;
+      for (int k = lane; k < ng1; k += 32) {
+        const double ex = P[3 * k] - tx, ey = P[3 * k + 1] - ty, ez = P[3 * k + 2] - tz;
+        const double d2 = ex * ex + ey * ey + ez * ez;
+        if (d2 < best) {
+          best = d2;
+          kb = k;
+        }
+      }
+      // the nearest point, the first of equally near ones
+      for (int o = 16; o > 0; o >>= 1) {
+        const double d2 = __shfl_xor_sync(0xffffffffu, best, o);
+        const int k = __shfl_xor_sync(0xffffffffu, kb, o);
+        if (k < ng1 && (kb == ng1 || d2 < best || (d2 == best && k < kb))) {
+          best = d2;
+          kb = k;
+        }
+      }
+      if (kb == ng1) continue;
+      if (lane == 0 && cnt < kNearMax) {
+        near_v[t * kNearMax + cnt] = (int)v;
+        near_k[t * kNearMax + cnt] = kb;
+      }
+      cnt++;
+    }
   }
+  if (lane) return;
+  count[t] = cnt <= kNearMax ? cnt : kNearMax + 1;
+  if (cnt > kNearMax) atomicMin(over, (unsigned long long)t);
+}
+
+// Recurrence tables of the normalised associated Legendre functions (near_tables): rows n = 0..p
+// of [3][32] (order m): a and b of P(m, n) = a x P(m, n - 1) - b P(m, n - 2), and c of the
+// derivative's P(m + 1, n) term; then [32] diagonal factors, P(m, m) = diag (-s)^m.
+__host__ __device__ constexpr int near_table_doubles(int p) { return 96 * (p + 1) + 32; }
+
+// Value, d/dtheta and d/dphi of the 3 functions S[3][nc] at (x = cos theta, phi), summed over the
+// G lanes of a group (all its lanes get them): lane m < p + 1 runs the recurrence of order m and
+// the order-m blocks (the reference's LegPoly / LegPolyDeriv, src/SphericalHarmonics.cc:889-950;
+// P(m + 1, n) for the derivative comes from lane m + 1).
+template <int G>
+__device__ __forceinline__ void sh_point(const double* __restrict__ S, const double* __restrict__ tab, int p,
+                                         const int* __restrict__ blk_off, double x, double phi, bool grads,
+                                         double* val) {
+  const int m = threadIdx.x & (G - 1);
+  const int nc = p * (p + 2);
+  const double s = sqrt(fmax(1.0 - x * x, 0.0)), si = s > 0.0 ? 1.0 / s : 0.0;
+  double pw = 1.0, b = -s;  // (-s)^m
+#pragma unroll
+  for (int i = 0; i < (G == 16 ? 4 : 5); i++) {
+    if (m >> i & 1) pw *= b;
+    b *= b;
+  }
+  const bool act = m <= p;
+  const double pmm = act ? tab[96 * (p + 1) + m] * pw : 0.0;
+  double cm = 1.0, sm = 0.0;
+  if (act) sincos(m * phi, &sm, &cm);
   const int jc = m == 0 ? 0 : (m == p ? 2 * p - 1 : 2 * m - 1);  // cos block of order m
-  const int js = (m >= 1 && m < p) ? 2 * m : -1;                  // sin block
-  const int oc = m <= p ? blk_off[jc] : 0, os = js >= 0 ? blk_off[js] : 0;
-  double pm2 = 0.0, pm1 = pmm;
+  const bool sine = m >= 1 && m < p;                              // it has a sin block
+  const double* Sc = S + (act ? blk_off[jc] : 0) - m;
+  const double* Ss = S + (sine ? blk_off[2 * m] : 0) - m;
+  double vc[3] = {0, 0, 0}, vs[3] = {0, 0, 0}, dc[3] = {0, 0, 0}, ds[3] = {0, 0, 0};
+  const double mx = m * x * si;
+  double pm2 = 0.0, pm1 = 0.0;
   for (int n = 0; n <= p; n++) {
-    double pn = 0.0;
-    if (m <= p && n >= m) {
-      if (n == m) {
-        pn = pmm;
-      } else {
-        const double a = sqrt(((2.0 * n - 1) * (2.0 * n + 1)) / ((double)(n - m) * (n + m)));
-        const double b = n > 1 ? sqrt(((2.0 * n + 1) * (n + m - 1) * (n - m - 1)) / ((double)(n - m) * (n + m) * (2 * n - 3)))
-                               : 0.0;
-        pn = x * a * pm1 - b * pm2;
-        pm2 = pm1;
-        pm1 = pn;
+    const double* row = tab + 96 * n + m;
+    const double pn = n == m ? pmm : n > m ? row[0] * x * pm1 - row[32] * pm2 : 0.0;
+    pm2 = pm1;
+    pm1 = pn;
+    const double pnext = __shfl_down_sync(0xffffffffu, pn, 1, G);
+    if (act && n >= m) {
+      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta)
+      const double dpn = s > 0.0 ? fma(mx, pn, row[64] * pnext) : 0.0;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const double a = Sc[d * nc + n];
+        vc[d] = fma(a, pn, vc[d]);
+        if (grads) dc[d] = fma(a, dpn, dc[d]);
+        if (sine) {
+          const double e = Ss[d * nc + n];
+          vs[d] = fma(e, pn, vs[d]);
+          if (grads) ds[d] = fma(e, dpn, ds[d]);
+        }
       }
     }
-    // P(m + 1, n) from the next lane (0 beyond the diagonal) for the theta derivative
-    const double pnext = __shfl_down_sync(0xffffffffu, pn, 1);
-    if (m <= p && n >= m) {
-      const double c2 = m + 1 <= n ? sqrt(n + m + 1.0) * sqrt((double)(n - m)) : 0.0;
-      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta)
-      const double dpn = s > 0.0 ? (m * x * pn + c2 * s * (m + 1 <= n ? pnext : 0.0)) / s : 0.0;
-      const int ic = oc + (n - m);
-      for (int d = 0; d < 3; d++) {
-        const double a = S[(long)d * nc + ic];
-        acc[d] += a * pn * cm;
-        if (grads) {
-          acc[3 + d] += a * dpn * cm;
-          acc[6 + d] += a * pn * dcm;
-        }
-      }
-      if (js >= 0) {
-        const int is = os + (n - m);
-        for (int d = 0; d < 3; d++) {
-          const double a = S[(long)d * nc + is];
-          acc[d] += a * pn * sm;
-          if (grads) {
-            acc[3 + d] += a * dpn * sm;
-            acc[6 + d] += a * pn * dsm;
-          }
-        }
-      }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    val[d] = fma(vc[d], cm, vs[d] * sm);
+    if (grads) {
+      val[3 + d] = fma(dc[d], cm, ds[d] * sm);
+      val[6 + d] = m * (vs[d] * cm - vc[d] * sm);
     }
   }
 #pragma unroll
   for (int i = 0; i < 9; i++) {
-    double v = acc[i];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (i >= 3 && !grads) break;
+    double v = val[i];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
     val[i] = kSqrt2Pi * v;
   }
 }
 
 struct NearArgs {
   const double* trg;
+  long M;
   const int* count;
   const int* near_v;
   const int* near_k;
+  const unsigned long long* rmax_bits;
   const double* Sx;      // [nv][3][nc] position coefficients
   const double* Vc;      // [nv][3][nc] self-velocity coefficients (single + double layer)
   const double* Gc;      // [nv][3][nc] double-layer density coefficients, or null
@@ -208,136 +241,176 @@ struct NearArgs {
   const double* nrm_up;  // null without a double layer
   const double* dden_up;
   const double* theta_up;  // [p_up + 1] latitudes of the upsampled grid
+  const double* tab;       // near_tables
   const int* blk_off;
   int p, p_up;
-  double r_near;
+  double* proj;  // [kNearMax M][10]: projection, unit direction, value there, |T - P| / r_near
   double* corr;  // [M][kNearMax][3]
 };
 
-// One CTA of 128 threads per (target, slot): warp 0 projects the target on the vesicle
-// and evaluates the on-surface values at the projection; then all threads sum the smooth
-// quadrature at the 7 line points and at the target; thread 0 writes the correction.
-__global__ void __launch_bounds__(128) k_near_correct(NearArgs A) {
-  const long t = blockIdx.x / kNearMax;
-  const int slot = blockIdx.x - (int)(t * kNearMax);
-  const int cnt = A.count[t];
-  if (slot >= cnt || cnt > kNearMax) return;
-  __shared__ double sh[8 * 3];   // line points (7) and the target
-  __shared__ double s_y0[3];     // on-surface value at the projection
-  __shared__ double s_x;         // |T - P| / r_near
-  __shared__ double red[4][8 * 3];
-  const int v = A.near_v[t * kNearMax + slot], k0 = A.near_k[t * kNearMax + slot];
-  const int p = A.p, nc = p * (p + 2), ng1 = 2 * A.p_up * (A.p_up + 1);
-  const double tx = A.trg[3 * t], ty = A.trg[3 * t + 1], tz = A.trg[3 * t + 2];
-  if (threadIdx.x < 32) {
-    const double* S = A.Sx + (long)v * 3 * nc;
-    double th = A.theta_up[k0 / (2 * A.p_up)], ph = M_PI * (k0 % (2 * A.p_up)) / A.p_up;
-    double val[9];
-    for (int itn = 0; itn < 40; itn++) {  // Gauss-Newton on |X(theta, phi) - T|^2
-      sh_point(S, p, A.blk_off, cos(th), ph, true, val);
-      const double rx = val[0] - tx, ry = val[1] - ty, rz = val[2] - tz;
-      const double a11 = val[3] * val[3] + val[4] * val[4] + val[5] * val[5];
-      const double a12 = val[3] * val[6] + val[4] * val[7] + val[5] * val[8];
-      const double a22 = val[6] * val[6] + val[7] * val[7] + val[8] * val[8];
-      const double g1 = val[3] * rx + val[4] * ry + val[5] * rz, g2 = val[6] * rx + val[7] * ry + val[8] * rz;
-      const double reg = 1e-14 * (a11 + a22);
-      const double b11 = a11 + reg, b22 = a22 + reg, det = b11 * b22 - a12 * a12;
-      const double d1 = -(b22 * g1 - a12 * g2) / det, d2 = -(b11 * g2 - a12 * g1) / det;
+constexpr int kProjWarps = 4;
+
+// Projection of each near target on its vesicle and the on-surface values there: one group of G
+// lanes per (slot, target) pair, slot-major (most targets have one near vesicle, so the groups in
+// use are neighbours). The vesicle's coefficients and the recurrence tables are staged in shared
+// memory. 0.64 ms for 15,000 pairs at p = 12; what bounds it is the serial chain of up to 40 Gauss-Newton steps of p + 1 recurrence
+// steps each: with the square roots and divisions of the recurrence in tables, 16 lanes per pair
+// at p <= 15 and every warp at it (one warp of a 128-thread CTA per pair, three waiting, and
+// the coefficients recomputed took 14.5 ms for 15,000 pairs at p = 12).
+template <int G>
+__global__ void __launch_bounds__(32 * kProjWarps) k_near_project(NearArgs A) {
+  extern __shared__ double smn[];
+  const int p = A.p, nc = p * (p + 2);
+  double* tab = smn;
+  int* bo = reinterpret_cast<int*>(tab + near_table_doubles(p));
+  double* Sall = tab + near_table_doubles(p) + p + 1;
+  const int grp = threadIdx.x / G, gl = threadIdx.x & (G - 1);
+  const long i = (long)blockIdx.x * (32 * kProjWarps / G) + grp;
+  const int slot = (int)(i / A.M);
+  const long t = i - (long)slot * A.M;
+  const int cnt = slot < kNearMax ? A.count[t] : 0;
+  const bool on = slot < cnt && cnt <= kNearMax;
+  if (__syncthreads_or(on) == 0) return;
+  for (int k = threadIdx.x; k < near_table_doubles(p); k += 32 * kProjWarps) tab[k] = A.tab[k];
+  for (int k = threadIdx.x; k <= 2 * p; k += 32 * kProjWarps) bo[k] = A.blk_off[k];
+  double* S = Sall + grp * 3 * nc;
+  const int v = on ? A.near_v[t * kNearMax + slot] : 0, k0 = on ? A.near_k[t * kNearMax + slot] : 0;
+  if (on)
+    for (int k = gl; k < 3 * nc; k += G) S[k] = A.Sx[(long)v * 3 * nc + k];
+  __syncthreads();
+  // the groups of a warp run their steps together (one finished early repeats nothing: its
+  // angles stay); an idle group follows on its staged (unused) values
+  const double tx = on ? A.trg[3 * t] : 0.0, ty = on ? A.trg[3 * t + 1] : 0.0, tz = on ? A.trg[3 * t + 2] : 0.0;
+  double th = A.theta_up[k0 / (2 * A.p_up)], ph = M_PI * (k0 % (2 * A.p_up)) / A.p_up;
+  double val[9];
+  const double* Sg = on ? S : A.Sx;
+  bool done = !on;
+  for (int itn = 0; itn < 40; itn++) {  // Gauss-Newton on |X(theta, phi) - T|^2
+    if (__all_sync(0xffffffffu, done)) break;
+    sh_point<G>(Sg, tab, p, bo, cos(th), ph, true, val);
+    const double rx = val[0] - tx, ry = val[1] - ty, rz = val[2] - tz;
+    const double a11 = val[3] * val[3] + val[4] * val[4] + val[5] * val[5];
+    const double a12 = val[3] * val[6] + val[4] * val[7] + val[5] * val[8];
+    const double a22 = val[6] * val[6] + val[7] * val[7] + val[8] * val[8];
+    const double g1 = val[3] * rx + val[4] * ry + val[5] * rz, g2 = val[6] * rx + val[7] * ry + val[8] * rz;
+    const double reg = 1e-14 * (a11 + a22);
+    const double b11 = a11 + reg, b22 = a22 + reg, det = b11 * b22 - a12 * a12;
+    const double d1 = -(b22 * g1 - a12 * g2) / det, d2 = -(b11 * g2 - a12 * g1) / det;
+    if (!done) {
       th += d1;
       ph += d2;
-      if (fmax(fabs(d1), fabs(d2)) < 1e-15) break;
     }
-    sh_point(S, p, A.blk_off, cos(th), ph, true, val);
-    const double px = val[0], py = val[1], pz = val[2];
-    // outward normal X_theta x X_phi (the orientation of the library's unit normals)
-    double nx = val[4] * val[8] - val[5] * val[7], ny = val[5] * val[6] - val[3] * val[8],
-           nz = val[3] * val[7] - val[4] * val[6];
-    const double nn = sqrt(nx * nx + ny * ny + nz * nz);
-    nx /= nn;
-    ny /= nn;
-    nz /= nn;
-    const double dx = tx - px, dy = ty - py, dz = tz - pz;
-    const double dist = sqrt(dx * dx + dy * dy + dz * dz);
-    const bool exterior = dx * nx + dy * ny + dz * nz >= 0.0;
-    double ux = nx, uy = ny, uz = nz;
-    if (dist > 0.0) {
-      ux = dx / dist;
-      uy = dy / dist;
-      uz = dz / dist;
-    }
-    double vs[9];
-    sh_point(A.Vc + (long)v * 3 * nc, p, A.blk_off, cos(th), ph, false, vs);
-    double y0[3] = {vs[0], vs[1], vs[2]};
-    if (A.Gc) {
-      double gs[9];
-      sh_point(A.Gc + (long)v * 3 * nc, p, A.blk_off, cos(th), ph, false, gs);
-      const double jump = exterior ? 0.5 : -0.5;
-      for (int d = 0; d < 3; d++) y0[d] += jump * gs[d];
-    }
-    if (threadIdx.x == 0) {
-      for (int l = 1; l < kInterpDeg; l++) {
-        const double r = A.r_near * inter_point(l);
-        sh[3 * (l - 1)] = px + r * ux;
-        sh[3 * (l - 1) + 1] = py + r * uy;
-        sh[3 * (l - 1) + 2] = pz + r * uz;
-      }
-      sh[21] = tx;
-      sh[22] = ty;
-      sh[23] = tz;
-      for (int d = 0; d < 3; d++) s_y0[d] = y0[d];
-      s_x = dist / A.r_near;
-    }
+    // at this length the steps are the rounding of the surface itself
+    done = done || fmax(fabs(d1), fabs(d2)) < kStepDone;
   }
-  __syncthreads();
-  // smooth upsampled quadrature of vesicle v at the 8 points
+  sh_point<G>(Sg, tab, p, bo, cos(th), ph, true, val);
+  const double px = val[0], py = val[1], pz = val[2];
+  // outward normal X_theta x X_phi (the orientation of the library's unit normals)
+  double nx = val[4] * val[8] - val[5] * val[7], ny = val[5] * val[6] - val[3] * val[8],
+         nz = val[3] * val[7] - val[4] * val[6];
+  const double nn = sqrt(nx * nx + ny * ny + nz * nz);
+  nx /= nn;
+  ny /= nn;
+  nz /= nn;
+  const double dx = tx - px, dy = ty - py, dz = tz - pz;
+  const double dist = sqrt(dx * dx + dy * dy + dz * dz);
+  const bool exterior = dx * nx + dy * ny + dz * nz >= 0.0;
+  double ux = nx, uy = ny, uz = nz;
+  if (dist > 0.0) {
+    ux = dx / dist;
+    uy = dy / dist;
+    uz = dz / dist;
+  }
+  double y0[9];
+  sh_point<G>(A.Vc + (long)v * 3 * nc, tab, p, bo, cos(th), ph, false, y0);
+  if (A.Gc) {
+    double gs[9];
+    sh_point<G>(A.Gc + (long)v * 3 * nc, tab, p, bo, cos(th), ph, false, gs);
+    const double jump = exterior ? 0.5 : -0.5;
+    for (int d = 0; d < 3; d++) y0[d] += jump * gs[d];
+  }
+  if (on && gl == 0) {
+    double* o = A.proj + 10 * i;
+    o[0] = px;
+    o[1] = py;
+    o[2] = pz;
+    o[3] = ux;
+    o[4] = uy;
+    o[5] = uz;
+    o[6] = y0[0];
+    o[7] = y0[1];
+    o[8] = y0[2];
+    o[9] = dist / near_radius(A.rmax_bits, A.p_up);
+  }
+}
+
+// The correction of each pair: one CTA of 128 threads sums the smooth upsampled quadrature of the
+// vesicle at the 7 line points and at the target; threads 0..2 interpolate. Bound by the FP64 pipe
+// (8 targets x 1,200 sources per pair; 0.54 ms for 15,000 pairs at p = 12).
+template <bool DL>
+__global__ void __launch_bounds__(128) k_near_correct(NearArgs A) {
+  const long i = blockIdx.x;
+  const int slot = (int)(i / A.M);
+  const long t = i - (long)slot * A.M;
+  const int cnt = A.count[t];
+  if (slot >= cnt || cnt > kNearMax) return;
+  __shared__ double red[4][8 * 3];
+  const int v = A.near_v[t * kNearMax + slot];
+  const int ng1 = 2 * A.p_up * (A.p_up + 1);
+  const double* o = A.proj + 10 * i;
+  const double r_near = near_radius(A.rmax_bits, A.p_up);
+  double pt[8][3];  // line points (7) and the target
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+#pragma unroll
+    for (int d = 0; d < 3; d++) pt[q][d] = q < 7 ? o[d] + r_near * inter_point(q + 1) * o[3 + d] : A.trg[3 * t + d];
   double acc[24];
 #pragma unroll
-  for (int i = 0; i < 24; i++) acc[i] = 0.0;
+  for (int k = 0; k < 24; k++) acc[k] = 0.0;
   const double* P = A.pos_up + 3 * (long)v * ng1;
   const double* D = A.den_up + 3 * (long)v * ng1;
-  const double* Nn = A.nrm_up ? A.nrm_up + 3 * (long)v * ng1 : nullptr;
-  const double* G = A.dden_up ? A.dden_up + 3 * (long)v * ng1 : nullptr;
+  const double* Nn = DL ? A.nrm_up + 3 * (long)v * ng1 : nullptr;
+  const double* Gd = DL ? A.dden_up + 3 * (long)v * ng1 : nullptr;
   for (int s = threadIdx.x; s < ng1; s += blockDim.x) {
     const double sx = P[3 * s], sy = P[3 * s + 1], sz = P[3 * s + 2];
     const double fx = D[3 * s], fy = D[3 * s + 1], fz = D[3 * s + 2];
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       // single layer: r = source - point (src/CPUKernels.cc:1011-1057)
-      const double rx = sx - sh[3 * q], ry = sy - sh[3 * q + 1], rz = sz - sh[3 * q + 2];
+      const double rx = sx - pt[q][0], ry = sy - pt[q][1], rz = sz - pt[q][2];
       const double r2 = rx * rx + ry * ry + rz * rz;
-      const double ri = r2 > 0.0 ? rsqrt_f64(r2) : 0.0;
-      const double c = (rx * fx + ry * fy + rz * fz) * ri * ri;
-      acc[3 * q] += (fx + c * rx) * ri * kInv8Pi;
-      acc[3 * q + 1] += (fy + c * ry) * ri * kInv8Pi;
-      acc[3 * q + 2] += (fz + c * rz) * ri * kInv8Pi;
-      if (Nn) {  // double layer: r = point - source, 3/(4 pi) (r.n)(r.g) r / |r|^5
-        const double rn = -(rx * Nn[3 * s] + ry * Nn[3 * s + 1] + rz * Nn[3 * s + 2]);
-        const double rg = -(rx * G[3 * s] + ry * G[3 * s + 1] + rz * G[3 * s + 2]);
-        const double w = kDl * rn * rg * ri * ri * ri * ri * ri;
-        acc[3 * q] -= w * rx;
-        acc[3 * q + 1] -= w * ry;
-        acc[3 * q + 2] -= w * rz;
+      double ri = rsqrt_f64_int_seed(r2);
+      ri = r2_in_range(r2) ? ri : 0.0;
+      const double ri2 = ri * ri;
+      double c = (rx * fx + ry * fy + rz * fz) * ri2 * ri;
+      if (DL) {  // double layer, r = point - source: 3/(4 pi) (r.n)(r.g) r / |r|^5, 6 times 1/(8 pi)
+        const double rn = rx * Nn[3 * s] + ry * Nn[3 * s + 1] + rz * Nn[3 * s + 2];
+        const double rg = rx * Gd[3 * s] + ry * Gd[3 * s + 1] + rz * Gd[3 * s + 2];
+        c -= 6.0 * rn * rg * (ri2 * ri2 * ri);
       }
+      acc[3 * q] = fma(c, rx, fma(fx, ri, acc[3 * q]));
+      acc[3 * q + 1] = fma(c, ry, fma(fy, ri, acc[3 * q + 1]));
+      acc[3 * q + 2] = fma(c, rz, fma(fz, ri, acc[3 * q + 2]));
     }
   }
   // fixed-order reduction: warp shuffles, then the 4 warps in order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < 24; i++) {
-    double a = acc[i];
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) red[warp][i] = a;
+  for (int k = 0; k < 24; k++) {
+    double a = acc[k];
+    for (int of = 16; of > 0; of >>= 1) a += __shfl_xor_sync(0xffffffffu, a, of);
+    if (lane == 0) red[warp][k] = a * kInv8Pi;
   }
   __syncthreads();
   if (threadIdx.x < 3) {
     const int d = threadIdx.x;
     double y[kInterpDeg];
-    y[0] = s_y0[d];
+    y[0] = o[6 + d];
     for (int l = 1; l < kInterpDeg; l++)
       y[l] = ((red[0][3 * (l - 1) + d] + red[1][3 * (l - 1) + d]) + (red[2][3 * (l - 1) + d] + red[3][3 * (l - 1) + d]));
     const double direct = (red[0][21 + d] + red[1][21 + d]) + (red[2][21 + d] + red[3][21 + d]);
     double interp = 0.0;
-    for (int l = 0; l < kInterpDeg; l++) interp += y[l] * inter_poly(s_x, l);
+    for (int l = 0; l < kInterpDeg; l++) interp += y[l] * inter_poly(o[9], l);
     A.corr[(t * kNearMax + slot) * 3 + d] = interp - direct;
   }
 }
@@ -363,28 +436,62 @@ int launch_centroid_radius(const double* X, long nv, int p, double* cen_r, unsig
   return VES3D_OK;
 }
 
+// Recurrence tables of k_near_project (see near_table_doubles).
+std::vector<double> near_tables(int p) {
+  std::vector<double> t(near_table_doubles(p), 0.0);
+  double d = 0.28209479177387814;  // 1/sqrt(4 pi)
+  for (int m = 0; m <= p; m++) {
+    if (m > 0) d *= std::sqrt((2.0 * m + 1.0) / (2.0 * m));
+    t[96 * (p + 1) + m] = d;
+    for (int n = m + 1; n <= p; n++) {
+      t[96 * n + m] = std::sqrt(((2.0 * n - 1) * (2.0 * n + 1)) / ((double)(n - m) * (n + m)));
+      if (n > m + 1)
+        t[96 * n + 32 + m] =
+            std::sqrt(((2.0 * n + 1) * (n + m - 1) * (n - m - 1)) / ((double)(n - m) * (n + m) * (2 * n - 3)));
+      t[96 * n + 64 + m] = std::sqrt(n + m + 1.0) * std::sqrt((double)(n - m));
+    }
+  }
+  return t;
+}
+
 int launch_near_find(const double* trg, long M, const double* cen_r, long nv, const double* pos_up, int p_up,
-                     double r_near, int* count, int* near_v, int* near_k, cudaStream_t st) {
+                     unsigned long long* rmax_over, int* count, int* near_v, int* near_k, cudaStream_t st) {
   if (M <= 0) return VES3D_OK;
-  k_near_find<<<(unsigned)((M + 127) / 128), 128, 0, st>>>(trg, M, cen_r, nv, pos_up, ngrid_(p_up), r_near, count,
-                                                          near_v, near_k);
+  VES3D_CK(cudaMemsetAsync(rmax_over + 1, 0xff, sizeof(unsigned long long), st));
+  k_near_find<<<(unsigned)((M + 3) / 4), 128, 0, st>>>(trg, M, cen_r, nv, pos_up, p_up, rmax_over, rmax_over + 1, count,
+                                                       near_v, near_k);
+  VES3D_LAUNCHED();
+  return VES3D_OK;
+}
+
+template <int G>
+static int launch_project(const NearArgs& a, cudaStream_t st) {
+  const int per = 32 * kProjWarps / G, p = a.p;
+  const size_t smem = ((size_t)near_table_doubles(p) + p + 1 + (size_t)per * 3 * p * (p + 2)) * sizeof(double);
+  VES3D_CK(cudaFuncSetAttribute(k_near_project<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_near_project<G><<<(unsigned)((a.M * kNearMax + per - 1) / per), 32 * kProjWarps, smem, st>>>(a);
   VES3D_LAUNCHED();
   return VES3D_OK;
 }
 
 int launch_near_correct(const double* trg, long M, const int* count, const int* near_v, const int* near_k,
-                        const double* Sx, const double* Vc, const double* Gc, const double* pos_up,
-                        const double* den_up, const double* nrm_up, const double* dden_up, const double* theta_up,
-                        const int* blk_off, int p, int p_up, double r_near, double* corr, double* vel,
-                        cudaStream_t st) {
+                        const unsigned long long* rmax_over, const double* Sx, const double* Vc, const double* Gc,
+                        const double* pos_up, const double* den_up, const double* nrm_up, const double* dden_up,
+                        const double* theta_up, const double* tab, const int* blk_off, int p, int p_up, double* proj,
+                        double* corr, double* vel, cudaStream_t st) {
   if (M <= 0) return VES3D_OK;
   if (p + 1 > 32) {
     set_error("near-singular correction: orders up to 31");
     return VES3D_ERR_ARG;
   }
-  NearArgs a{trg, count, near_v, near_k, Sx, Vc, Gc, pos_up, den_up, nrm_up, dden_up, theta_up, blk_off,
-             p, p_up, r_near, corr};
-  k_near_correct<<<(unsigned)(M * kNearMax), 128, 0, st>>>(a);
+  const NearArgs a{trg, M, count, near_v, near_k, rmax_over, Sx, Vc, Gc, pos_up, den_up, nrm_up, dden_up, theta_up,
+                   tab, blk_off, p, p_up, proj, corr};
+  const int s = p + 1 <= 16 ? launch_project<16>(a, st) : launch_project<32>(a, st);
+  if (s) return s;
+  if (nrm_up)
+    k_near_correct<true><<<(unsigned)(M * kNearMax), 128, 0, st>>>(a);
+  else
+    k_near_correct<false><<<(unsigned)(M * kNearMax), 128, 0, st>>>(a);
   VES3D_LAUNCHED();
   k_near_add<<<(unsigned)((M + 127) / 128), 128, 0, st>>>(count, corr, M, vel);
   VES3D_LAUNCHED();

@@ -203,17 +203,17 @@ struct ves3d_sv {
   bool near_on = false;
   double *nu_X = nullptr, *nu_Xt = nullptr, *nu_Xp = nullptr, *nu_F = nullptr, *nu_G = nullptr, *nu_area = nullptr;
   double *nu_pos = nullptr, *nu_den = nullptr, *nu_nrm = nullptr, *nu_dden = nullptr, *nu_cen = nullptr;
-  double *nu_theta = nullptr, *nu_w = nullptr, *nu_corr = nullptr;
-  unsigned long long* nu_rmax = nullptr;
+  double *nu_theta = nullptr, *nu_w = nullptr, *nu_corr = nullptr, *nu_proj = nullptr, *nu_tab = nullptr;
+  unsigned long long* nu_rmax = nullptr;  // largest radius, first target with too many near vesicles
   int *nu_count = nullptr, *nu_v = nullptr, *nu_k = nullptr;
   long nu_ves_cap = 0, nu_trg_cap = 0;
   double near_r = 0.0;  // r_near of the last corrected evaluation
   void free_near() {
     double* ps[] = {nu_X, nu_Xt, nu_Xp, nu_F, nu_G, nu_area, nu_pos, nu_den, nu_nrm, nu_dden, nu_cen, nu_theta, nu_w,
-                    nu_corr};
+                    nu_corr, nu_proj, nu_tab};
     for (double* q : ps) dfree(q);
     nu_X = nu_Xt = nu_Xp = nu_F = nu_G = nu_area = nu_pos = nu_den = nu_nrm = nu_dden = nu_cen = nullptr;
-    nu_theta = nu_w = nu_corr = nullptr;
+    nu_theta = nu_w = nu_corr = nu_proj = nu_tab = nullptr;
     dfree(nu_rmax);
     dfree(nu_count);
     dfree(nu_v);
@@ -744,7 +744,7 @@ int eval_trg_near(ves3d_sv* sv) {
   if ((s = run_self_apply(sv, dl))) return s;  // Fc (Gc) and the self coefficients Vc
   if (sv->nu_ves_cap < nv || (dl && !sv->nu_G)) {
     double* ps[] = {sv->nu_X, sv->nu_Xt, sv->nu_Xp, sv->nu_F, sv->nu_G, sv->nu_area, sv->nu_pos, sv->nu_den,
-                    sv->nu_nrm, sv->nu_dden, sv->nu_cen, sv->nu_theta, sv->nu_w};
+                    sv->nu_nrm, sv->nu_dden, sv->nu_cen, sv->nu_theta, sv->nu_w, sv->nu_tab};
     for (double* x : ps) dfree(x);
     const size_t f = (size_t)nv * 3 * ng1;
     s = 0;
@@ -759,7 +759,7 @@ int eval_trg_near(ves3d_sv* sv) {
     s |= dalloc(&sv->nu_nrm, f);
     s |= dalloc(&sv->nu_dden, f);
     s |= dalloc(&sv->nu_cen, 4 * (size_t)nv);
-    if (!sv->nu_rmax) s |= dalloc(&sv->nu_rmax, 1);
+    if (!sv->nu_rmax) s |= dalloc(&sv->nu_rmax, 2);
     // the upsampled grid's latitudes and smooth weights (LegendreWeights(p_up))
     std::vector<double> x, w, th(q + 1), sw(q + 1);
     gauss_legendre(q + 1, x, w);
@@ -769,6 +769,7 @@ int eval_trg_near(ves3d_sv* sv) {
     }
     if (!s) s = dupload(&sv->nu_theta, th, st);
     if (!s) s = dupload(&sv->nu_w, sw, st);
+    if (!s) s = dupload(&sv->nu_tab, near_tables(p), st);
     if (s) {
       sv->free_near();
       return s;
@@ -780,13 +781,15 @@ int eval_trg_near(ves3d_sv* sv) {
     dfree(sv->nu_v);
     dfree(sv->nu_k);
     dfree(sv->nu_corr);
+    dfree(sv->nu_proj);
     sv->nu_count = sv->nu_v = sv->nu_k = nullptr;
-    sv->nu_corr = nullptr;
+    sv->nu_corr = sv->nu_proj = nullptr;
     s = 0;
     s |= dalloc(&sv->nu_count, (size_t)M);
     s |= dalloc(&sv->nu_v, (size_t)M * kNearMax);
     s |= dalloc(&sv->nu_k, (size_t)M * kNearMax);
     s |= dalloc(&sv->nu_corr, (size_t)M * kNearMax * 3);
+    s |= dalloc(&sv->nu_proj, (size_t)M * kNearMax * 10);
     if (s) {
       sv->free_near();
       return s;
@@ -814,30 +817,28 @@ int eval_trg_near(ves3d_sv* sv) {
   if ((s = launch_targets_f64(sv->nu_pos, sv->nu_den, dl ? sv->nu_nrm : nullptr, dl ? sv->nu_dden : nullptr,
                               nv * ng1, sv->trg, M, sv->vtrg, sv->trg_part, st)))
     return s;
-  // r_near = r_ves 2 / sqrt(p_up) (src/NearSingular.cc:160, :119-158)
+  // r_near = r_ves 2 / sqrt(p_up) (src/NearSingular.cc:160, :119-158), formed where it is used
   if ((s = launch_centroid_radius(sv->X, nv, p, sv->nu_cen, sv->nu_rmax, st))) return s;
-  unsigned long long bits = 0;
-  VES3D_CK(cudaMemcpyAsync(&bits, sv->nu_rmax, sizeof(bits), cudaMemcpyDeviceToHost, st));
-  VES3D_CK(cudaStreamSynchronize(st));
-  double r_ves;
-  std::memcpy(&r_ves, &bits, sizeof(double));
-  sv->near_r = r_ves * 2.0 / std::sqrt((double)q);
-  if ((s = launch_near_find(sv->trg, M, sv->nu_cen, nv, sv->nu_pos, q, sv->near_r, sv->nu_count, sv->nu_v, sv->nu_k,
+  if ((s = launch_near_find(sv->trg, M, sv->nu_cen, nv, sv->nu_pos, q, sv->nu_rmax, sv->nu_count, sv->nu_v, sv->nu_k,
                             st)))
     return s;
-  {  // more near vesicles than slots for some target: an error, not a silent truncation
-    std::vector<int> c(M);
-    VES3D_CK(cudaMemcpyAsync(c.data(), sv->nu_count, M * sizeof(int), cudaMemcpyDeviceToHost, st));
-    VES3D_CK(cudaStreamSynchronize(st));
-    for (long t = 0; t < M; t++)
-      if (c[t] > kNearMax) {
-        set_error("target %ld is near more than %d vesicles (the near-singular correction's limit)", t, kNearMax);
-        return VES3D_ERR_ARG;
-      }
+  if ((s = launch_near_correct(sv->trg, M, sv->nu_count, sv->nu_v, sv->nu_k, sv->nu_rmax, sv->Sx, sv->Vc,
+                               dl ? sv->Gc : nullptr, sv->nu_pos, sv->nu_den, dl ? sv->nu_nrm : nullptr,
+                               dl ? sv->nu_dden : nullptr, sv->nu_theta, sv->nu_tab, T.blk_off, p, q, sv->nu_proj,
+                               sv->nu_corr, sv->vtrg, st)))
+    return s;
+  unsigned long long rmax_over[2] = {0, 0};
+  VES3D_CK(cudaMemcpyAsync(rmax_over, sv->nu_rmax, sizeof(rmax_over), cudaMemcpyDeviceToHost, st));
+  VES3D_CK(cudaStreamSynchronize(st));
+  double r_ves;
+  std::memcpy(&r_ves, &rmax_over[0], sizeof(double));
+  sv->near_r = r_ves * 2.0 / std::sqrt((double)q);
+  if (rmax_over[1] != ~0ull) {  // more near vesicles than slots: an error, not a silent truncation
+    set_error("target %ld is near more than %d vesicles (the near-singular correction's limit)", (long)rmax_over[1],
+              kNearMax);
+    return VES3D_ERR_ARG;
   }
-  return launch_near_correct(sv->trg, M, sv->nu_count, sv->nu_v, sv->nu_k, sv->Sx, sv->Vc, dl ? sv->Gc : nullptr,
-                             sv->nu_pos, sv->nu_den, dl ? sv->nu_nrm : nullptr, dl ? sv->nu_dden : nullptr,
-                             sv->nu_theta, T.blk_off, p, q, sv->near_r, sv->nu_corr, sv->vtrg, st);
+  return VES3D_OK;
 }
 
 }  // namespace
