@@ -416,9 +416,10 @@ __global__ void __launch_bounds__(RtItemCfg<P, TV>::NT, RtItemCfg<P, TV>::MINB)
   const int po = __ldg(T.perm_off + n), bn = __ldg(T.perm_off + n + 1) - po;
   const TV* M0 = active ? sM + sMo[n] + (sDm[c0] - po) * (bn | 1) : sM;
   const TV* M1 = c1 >= 0 ? sM + sMo[n] + (sDm[c1] - po) * (bn | 1) : M0;
-  for (int pole = 0; pole < 2; pole++) {
+  for (int pc = blockIdx.z; pc < 12; pc += gridDim.z) {
+    const int pole = pc / 6, comp = pc - 6 * pole;
     const int grid0 = pole == 0 ? t * 2 * P : (P - t) * 2 * P + P;
-    for (int comp = 0; comp < 6; comp++) {
+    {
       __syncthreads();
       // stage: A[j][dm(c)] = C[v][t][j][pole][comp][c], eight loads in flight per thread
       for (int i0 = tid; i0 < P * nc; i0 += NT * 8) {
@@ -496,7 +497,11 @@ static size_t rt_item_smem(int p0, int mpt) {
 template <int P, typename TC, typename TV = float>
 static int launch_rt_item(const TC* C, long nv, const DevTables& T, TV* SL3, cudaStream_t st) {
   const int mpt = mr_per_t(T);
-  dim3 grid(P + 1, (unsigned)nv);
+  // few vesicles: the 12 (pole, component) planes of a (vesicle, rotation) over several CTAs, up to
+  // four per SM (each plane's arithmetic stays as it is)
+  int planes = 1;
+  while (planes < 12 && (P + 1) * nv * planes < 4 * 148) planes = planes < 4 ? planes + 1 : planes == 4 ? 6 : 12;
+  dim3 grid(P + 1, (unsigned)nv, (unsigned)planes);
   const size_t smem = rt_item_smem<TV>(P, mpt);  // about 48 KB at p = 16 (four CTAs per SM), 149 KB at p = 24
   VES3D_CK(cudaFuncSetAttribute(k_rotate_transpose_item<P, TC, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)smem));
@@ -692,9 +697,21 @@ __global__ void __launch_bounds__(256, 2) k_rotate_transpose_tc(const double* __
 int launch_rotate_transpose_scatter(const double* C, long nv, const DevTables& T, double* SL3, cudaStream_t st) {
   if (nv <= 0) return VES3D_OK;
   const int p0 = T.p0, nc = ncoef_(p0);
-  // p = 16: the per-item kernel in FP64 (5.8 ms per 512-vesicle build against 9.5 ms for the
-  // DMMA form below, which keeps the other orders up to 16)
-  if (p0 == 16 && !tc_rotate_disabled()) return launch_rt_item<16, double, double>(C, nv, T, SL3, st);
+  // the per-item kernel in FP64 at its even orders (p = 16: 5.8 ms per 512-vesicle build against
+  // 9.5 ms for the DMMA form below, which keeps the odd orders; p = 12, 8 vesicles: 51 against 128 us;
+  // whole builds of 27 vesicles at p = 4 38 against 54 us, p = 20 4.9 against 7.6 ms)
+  if (!tc_rotate_disabled()) switch (p0) {
+      case 4: return launch_rt_item<4, double, double>(C, nv, T, SL3, st);
+      case 6: return launch_rt_item<6, double, double>(C, nv, T, SL3, st);
+      case 8: return launch_rt_item<8, double, double>(C, nv, T, SL3, st);
+      case 10: return launch_rt_item<10, double, double>(C, nv, T, SL3, st);
+      case 12: return launch_rt_item<12, double, double>(C, nv, T, SL3, st);
+      case 14: return launch_rt_item<14, double, double>(C, nv, T, SL3, st);
+      case 16: return launch_rt_item<16, double, double>(C, nv, T, SL3, st);
+      case 18: return launch_rt_item<18, double, double>(C, nv, T, SL3, st);
+      case 20: return launch_rt_item<20, double, double>(C, nv, T, SL3, st);
+      default: break;
+    }
   {
     // tensor-core form: the largest component block (3, 2 or 1 components x p0 rows)
     // whose staging fits two CTAs per SM; 6 must be a multiple of the block
