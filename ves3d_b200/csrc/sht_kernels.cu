@@ -52,55 +52,86 @@ __global__ void __launch_bounds__(256) k_analysis(const double* __restrict__ in,
   }
 }
 
+// FB functions per CTA. The Legendre sums take lanes along the latitudes (consecutive table
+// values, one coefficient broadcast) and one table value for the CTA's functions; the DFT takes lanes
+// along the longitudes, four latitudes per thread on one table value. Bound by the table reads from
+// L1: a load per multiply-add before (1,536 functions of p = 16: 260 us), one per FB or four now (71 us).
+template <int FB>
 __global__ void __launch_bounds__(256) k_synthesis(const double* __restrict__ S, long nfun, int nci, int nfi,
                                                    int nlat, int nlon, const double* __restrict__ leg,
                                                    const double* __restrict__ dleg,
                                                    const double* __restrict__ four,
                                                    const double* __restrict__ dfour,
-                                                   const int* __restrict__ blk_off, int fpb,
+                                                   const int* __restrict__ blk_off,
                                                    double* __restrict__ X, double* __restrict__ Xt,
                                                    double* __restrict__ Xp) {
-  extern __shared__ double sm[];
-  double* ss = sm;                                  // fpb * nci
-  double* sb = ss + (size_t)fpb * nci;              // fpb * nlat * nfi
-  double* sd = sb + (size_t)fpb * nlat * nfi;       // fpb * nlat * nfi (if Xp)
-  const long f0 = (long)blockIdx.x * fpb;
-  const int nf = (int)min((long)fpb, nfun - f0);
-  for (int i = threadIdx.x; i < nf * nci; i += blockDim.x) ss[i] = S[f0 * nci + i];
+  extern __shared__ __align__(16) double sm[];
+  const int nls = (nlat + 3) & ~3;                  // latitudes padded to whole groups of four
+  double* sb = sm;                                  // [FB][nfi][nls]
+  double* sd = sb + (size_t)FB * nfi * nls;         // the same of dleg (if Xp)
+  double* ss = sd + (Xp ? (size_t)FB * nfi * nls : 0);  // [FB][nci]
+  const long f0 = (long)blockIdx.x * FB;
+  const int nf = (int)min((long)FB, nfun - f0);
+  for (int i = threadIdx.x; i < FB * nci; i += blockDim.x) ss[i] = i < nf * nci ? S[f0 * nci + i] : 0.0;
   __syncthreads();
-  const int totB = nf * nlat * nfi;
-  for (int i = threadIdx.x; i < totB; i += blockDim.x) {
-    const int k = i % nfi, lat = (i / nfi) % nlat, f = i / (nfi * nlat);
-    const int c0 = __ldg(blk_off + k), c1 = __ldg(blk_off + k + 1);
-    const double* sr = ss + (size_t)f * nci;
-    double s = 0.0, d = 0.0;
-    for (int c = c0; c < c1; c++) {
-      s = fma(sr[c], __ldg(leg + (size_t)c * nlat + lat), s);
-      if (Xp) d = fma(sr[c], __ldg(dleg + (size_t)c * nlat + lat), d);
+  for (int i = threadIdx.x; i < nfi * nls; i += blockDim.x) {
+    const int k = i / nls, lat = i - k * nls;
+    double s[FB], d[FB];
+#pragma unroll
+    for (int f = 0; f < FB; f++) s[f] = d[f] = 0.0;
+    if (lat < nlat) {
+      const int c0 = __ldg(blk_off + k), c1 = __ldg(blk_off + k + 1);
+#pragma unroll 4
+      for (int c = c0; c < c1; c++) {
+        const double l = __ldg(leg + (size_t)c * nlat + lat), dl = Xp ? __ldg(dleg + (size_t)c * nlat + lat) : 0.0;
+#pragma unroll
+        for (int f = 0; f < FB; f++) {
+          s[f] = fma(ss[f * nci + c], l, s[f]);
+          d[f] = fma(ss[f * nci + c], dl, d[f]);
+        }
+      }
     }
-    sb[i] = s;
-    if (Xp) sd[i] = d;
+#pragma unroll
+    for (int f = 0; f < FB; f++) {
+      sb[f * nfi * nls + i] = s[f];
+      if (Xp) sd[f * nfi * nls + i] = d[f];
+    }
   }
   __syncthreads();
-  const int totX = nf * nlat * nlon;
-  for (int i = threadIdx.x; i < totX; i += blockDim.x) {
-    const int j = i % nlon, r = i / nlon;  // r = f*nlat + lat
-    const double* br = sb + (size_t)r * nfi;
-    double x = 0.0, xt = 0.0;
+  const int ngr = nls / 4;
+  for (int i = threadIdx.x; i < nf * ngr * nlon; i += blockDim.x) {
+    const int j = i % nlon, r = i / nlon, f = r / ngr, lat0 = 4 * (r - f * ngr);
+    const double* br = sb + (size_t)f * nfi * nls + lat0;
+    const double* dr = sd + (size_t)f * nfi * nls + lat0;
+    double x[4] = {0, 0, 0, 0}, xt[4] = {0, 0, 0, 0}, xp[4] = {0, 0, 0, 0};
 #pragma unroll 4
     for (int k = 0; k < nfi; k++) {
-      x = fma(br[k], __ldg(four + k * nlon + j), x);
-      if (Xt) xt = fma(br[k], __ldg(dfour + k * nlon + j), xt);
+      const double w = __ldg(four + k * nlon + j), dw = Xt ? __ldg(dfour + k * nlon + j) : 0.0;
+      const double2 b0 = *reinterpret_cast<const double2*>(br + k * nls);
+      const double2 b1 = *reinterpret_cast<const double2*>(br + k * nls + 2);
+      const double b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+      for (int l = 0; l < 4; l++) x[l] = fma(b[l], w, x[l]);
+      if (Xt)
+#pragma unroll
+        for (int l = 0; l < 4; l++) xt[l] = fma(b[l], dw, xt[l]);
+      if (Xp) {
+        const double2 d0 = *reinterpret_cast<const double2*>(dr + k * nls);
+        const double2 d1 = *reinterpret_cast<const double2*>(dr + k * nls + 2);
+        xp[0] = fma(d0.x, w, xp[0]);
+        xp[1] = fma(d0.y, w, xp[1]);
+        xp[2] = fma(d1.x, w, xp[2]);
+        xp[3] = fma(d1.y, w, xp[3]);
+      }
     }
-    X[f0 * nlat * nlon + i] = x;
-    if (Xt) Xt[f0 * nlat * nlon + i] = xt;
-    if (Xp) {
-      const double* dr = sd + (size_t)r * nfi;
-      double xp = 0.0;
-#pragma unroll 4
-      for (int k = 0; k < nfi; k++) xp = fma(dr[k], __ldg(four + k * nlon + j), xp);
-      Xp[f0 * nlat * nlon + i] = xp;
-    }
+#pragma unroll
+    for (int l = 0; l < 4; l++)
+      if (lat0 + l < nlat) {
+        const size_t o = ((size_t)(f0 + f) * nlat + lat0 + l) * nlon + j;
+        X[o] = x[l];
+        if (Xt) Xt[o] = xt[l];
+        if (Xp) Xp[o] = xp[l];
+      }
   }
 }
 
@@ -135,14 +166,16 @@ int launch_synthesis(const double* S, long nfun, int p0, int q, const double* le
                      const double* four, const double* dfour, const int* blk_off, double* X, double* Xt,
                      double* Xp, cudaStream_t st) {
   if (nfun <= 0) return VES3D_OK;
-  const int nci = ncoef_(p0), nfi = 2 * p0, nlat = q + 1, nlon = 2 * q;
-  const size_t per = (size_t)nci + (size_t)nlat * nfi * (Xp ? 2 : 1);
-  const int fpb = pick_fpb(per, nfun);
-  size_t smem = (size_t)fpb * per * sizeof(double);
-  if (smem > 48 * 1024) VES3D_CK(cudaFuncSetAttribute(k_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  long nblk = (nfun + fpb - 1) / fpb;
-  k_synthesis<<<(unsigned)nblk, 256, smem, st>>>(S, nfun, nci, nfi, nlat, nlon, leg, dleg, four, dfour, blk_off,
-                                                  fpb, X, Xt, Xp);
+  const int nci = ncoef_(p0), nfi = 2 * p0, nlat = q + 1, nlon = 2 * q, nls = (nlat + 3) & ~3;
+  const size_t per = ((size_t)nci + (size_t)nls * nfi * (Xp ? 2 : 1)) * sizeof(double);
+  // functions per CTA: as many as leave two CTAs per SM to run and 96 KB to a CTA
+  int fb = 4;
+  while (fb > 1 && (nfun < 2L * 148 * fb || per * fb > 96 * 1024)) fb /= 2;
+  const size_t smem = per * fb;
+  auto kernel = fb == 4 ? k_synthesis<4> : fb == 2 ? k_synthesis<2> : k_synthesis<1>;
+  if (smem > 48 * 1024) VES3D_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<(unsigned)((nfun + fb - 1) / fb), 256, smem, st>>>(S, nfun, nci, nfi, nlat, nlon, leg, dleg, four, dfour,
+                                                              blk_off, X, Xt, Xp);
   VES3D_LAUNCHED();
   return VES3D_OK;
 }
