@@ -47,6 +47,10 @@ int launch_grid2shc(const double* in, long nfun, int p, const double* four, cons
 // The same for FP32 grid values (FP64 arithmetic and output), p in {4, 8, 12, 16}.
 int launch_grid2shc_f32(const float* in, long nfun, int p, const double* four, const double* leg, const int* jf,
                         double* out, cudaStream_t st);
+// The stand-alone transforms at one order with their tables formed on chip (sht_fused_kernels.cu):
+// mode 0 analysis, 1 synthesis, 2 analysis, scale[degree] and synthesis (in place allowed).
+bool sht_fused_supported(int p);
+int launch_sht_fused(int mode, const double* in, long nfun, int p, const double* scale, double* out, cudaStream_t st);
 // shc_out[f][c] = shc_in[f][c] * scale[c] for nfun functions of nc coefficients
 int launch_scale_freq(const double* in, long nfun, int nc, const double* scale, double* out, cudaStream_t st);
 // SHC2Pole: P[2 f + t] = values of function f at x = -1 (t = 0) and x = +1 (t = 1) from its

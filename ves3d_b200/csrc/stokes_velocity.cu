@@ -1329,6 +1329,13 @@ int ves3d_sht_forward(const double* X, long n_fun, int p0, int p1, double* S, vo
   VES3D_ARG(p0 >= 1 && p1 >= 1 && p0 <= 128 && p1 <= 128, "orders must be in [1, 128]");
   VES3D_ARG(n_fun >= 0, "n_fun < 0");
   cudaStream_t st = (cudaStream_t)stream;
+  if (p0 == p1 && sht_fused_supported(p0)) {
+    const int s = launch_sht_fused(0, X, n_fun, p0, nullptr, S, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (s) return s;
+    VES3D_CK(e);
+    return VES3D_OK;
+  }
   AnalysisTables A;
   build_analysis_tables(p0, p1, A);
   std::vector<int> blk, jf;
@@ -1355,6 +1362,13 @@ int ves3d_sht_backward(const double* S, long n_fun, int p0, int p1, double* X, d
   VES3D_ARG(p0 >= 1 && p1 >= 1 && p0 <= 128 && p1 <= 128, "orders must be in [1, 128]");
   VES3D_ARG(n_fun >= 0, "n_fun < 0");
   cudaStream_t st = (cudaStream_t)stream;
+  if (p0 == p1 && !X_theta && !X_phi && sht_fused_supported(p0)) {
+    const int s = launch_sht_fused(1, S, n_fun, p0, nullptr, X, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (s) return s;
+    VES3D_CK(e);
+    return VES3D_OK;
+  }
   SynthTables syn;
   build_synth_tables(p0, p1, syn);
   std::vector<int> blk, jf;
@@ -1500,6 +1514,14 @@ int ves3d_sht_lowpass(const double* in, long n_fun, int p, int filter_freq, doub
   int s = ves3d_sht_filter_coeffs(p, filter_freq, exponent, coeff.data());
   if (s) return s;
   cudaStream_t st = (cudaStream_t)stream;
+  if (sht_fused_supported(p)) {
+    // coeff depends on the degree alone: the m = 0 block's values
+    s = launch_sht_fused(2, in, n_fun, p, coeff.data(), out, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (s) return s;
+    VES3D_CK(e);
+    return VES3D_OK;
+  }
   double *dc = nullptr, *shc = nullptr;
   if ((s = dupload(&dc, coeff, st))) return s;
   if ((s = dalloc(&shc, (size_t)n_fun * nc))) {
