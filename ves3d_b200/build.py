@@ -9,10 +9,11 @@ LIB = os.path.join(HERE, "libves3d_b200.so")
 # the benchmark's FMA-throughput probe, a separate library (not part of the product)
 PEAK_LIB = os.path.join(HERE, "libves3d_peak.so")
 PEAK_SOURCE = "peak_probe.cu"
-SOURCES = ["sh_tables.cc", "sht_kernels.cu", "sht_fused_kernels.cu", "singular_kernels.cu",
-           "direct_kernels.cu", "far_kernels.cu", "far_sym_kernels.cu", "build_kernels.cu",
-           "ring_kernels.cu", "stokes_velocity.cu", "noalloc.cu", "geometry_kernels.cu",
-           "bicgstab.cu", "mlp.cu", "device_prims.cu", "vtk_output.cu", "near_kernels.cu"]
+SOURCES = ["sh_tables.cc", "sht_kernels.cu", "sht_fused_kernels.cu", "grid2shc_kernels.cu",
+           "singular_kernels.cu", "direct_kernels.cu", "far_kernels.cu", "far_sym_kernels.cu",
+           "build_kernels.cu", "ring_kernels.cu", "stokes_velocity.cu", "noalloc.cu",
+           "geometry_kernels.cu", "bicgstab.cu", "mlp.cu", "device_prims.cu", "vtk_output.cu",
+           "near_kernels.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "-Wno-deprecated-gpu-targets"]
 

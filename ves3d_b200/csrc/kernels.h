@@ -40,11 +40,19 @@ typedef int (*MatVecFn)(void* ctx, const double* x, double* y);
 
 int launch_analysis(const double* in, long nfun, int pin, int pout, const double* four, const double* leg,
                     const int* jf, double* out, cudaStream_t st);
-// Grid2SHC(p, p): tensor-core kernel where instantiated (2p % 8 == 0), generic otherwise;
-// VES3D_TC_ANALYSIS=0 forces the generic kernel.
+// Grid2SHC(p, p) with the dense DFT (tensor cores where instantiated), for the position coefficients:
+// the mixed form's FP32 build stages turn their last bits into FP32 roundings (5e-8 at single points
+// of 512 vesicles), so they keep one order of operations.
+int launch_grid2shc_dense(const double* in, long nfun, int p, const double* four, const double* leg, const int* jf,
+                          double* out, cudaStream_t st);
+// Grid2SHC(p, p): the folded kernel (grid2shc_kernels.cu) at the orders it is instantiated for, the
+// dense forms otherwise; VES3D_TC_ANALYSIS=0 forces the generic kernel.
+bool grid2shc_folded(int p);
+int launch_grid2shc_folded(const double* in, long nfun, int p, const double* leg, const int* jf, double* out,
+                           cudaStream_t st);
 int launch_grid2shc(const double* in, long nfun, int p, const double* four, const double* leg, const int* jf,
                     double* out, cudaStream_t st);
-// The same for FP32 grid values (FP64 arithmetic and output), p in {4, 8, 12, 16}.
+// The same for FP32 grid values in FP32 (FP64 output), p in {12, 16, 24}.
 int launch_grid2shc_f32(const float* in, long nfun, int p, const double* four, const double* leg, const int* jf,
                         double* out, cudaStream_t st);
 // The stand-alone transforms at one order with their tables formed on chip (sht_fused_kernels.cu):

@@ -938,7 +938,7 @@ int ves3d_sv_set_src_coord(ves3d_sv* sv, const double* S, long n_ves, int is_dev
     VES3D_CK(cudaStreamSynchronize(sv->stream));
     sv->off_nves = n_ves;
   }
-  if ((s = launch_grid2shc(sv->X, n_ves * 3, p0, T.ana_four, T.ana_leg, T.jf_of_coef, sv->Sx, sv->stream)))
+  if ((s = launch_grid2shc_dense(sv->X, n_ves * 3, p0, T.ana_four, T.ana_leg, T.jf_of_coef, sv->Sx, sv->stream)))
     return s;
   if ((s = launch_synthesis(sv->Sx, n_ves * 3, p0, p0, T.syn0_leg, T.syn0_dleg, T.syn0_four, T.syn0_dfour, T.blk_off,
                             sv->Vself /* scratch: filtered grid, unused */, sv->Xt, sv->Xp, sv->stream)))
