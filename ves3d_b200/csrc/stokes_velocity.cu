@@ -267,7 +267,12 @@ struct ves3d_sv {
     graph = nullptr;
   }
   cudaEvent_t pc_ev[3 + kPcStreams] = {};
-  cudaEvent_t ev[10] = {};
+  // ev: [0, 1] self-matrix build, [2, 3] self apply, [4, 5] far field, [6] end of the evaluation,
+  // [8, 9] far double layer, [10, 11] double-layer build. Their times are read when asked for, or
+  // where the call waits for its result anyway (collect_times): the host queues a whole evaluation
+  // without stopping between its stages.
+  cudaEvent_t ev[12] = {}, ev_copied = nullptr;
+  bool t_setup = false, t_setup_dl = false, t_eval = false, t_eval_dl = false, check_tc = false;
   float ms[4] = {0, 0, 0, 0};
   float far_dl_ms = 0;  // the far double layer's segment kernels in the last evaluation
 
@@ -289,6 +294,7 @@ struct ves3d_sv {
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
     tab.reset();
+    if (ev_copied) cudaEventDestroy(ev_copied);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_built) cudaEventDestroy(ev_built);
@@ -509,10 +515,44 @@ int copy_out(double* dst, const double* src, size_t n, int is_device, cudaStream
 }
 
 int alloc_scratch(ves3d_sv* sv);
-int run_setup(ves3d_sv* sv, bool dl = false);
+int run_setup(ves3d_sv* sv, bool dl = false, bool wait = true);
+
+// Wait for the timed stages that were queued and take their times; with the tensor-core build, its
+// error flag.
+int collect_times(ves3d_sv* sv) {
+  if (sv->t_eval) {
+    VES3D_CK(cudaEventSynchronize(sv->ev[6]));
+    VES3D_CK(cudaEventElapsedTime(&sv->ms[1], sv->ev[2], sv->ev[3]));
+    VES3D_CK(cudaEventElapsedTime(&sv->ms[2], sv->ev[4], sv->ev[5]));
+    VES3D_CK(cudaEventElapsedTime(&sv->ms[3], sv->ev[2], sv->ev[6]));
+    sv->far_dl_ms = 0;
+    if (sv->t_eval_dl) VES3D_CK(cudaEventElapsedTime(&sv->far_dl_ms, sv->ev[8], sv->ev[9]));
+    sv->t_eval = false;
+  }
+  if (sv->t_setup) {
+    VES3D_CK(cudaEventSynchronize(sv->ev[1]));
+    VES3D_CK(cudaEventElapsedTime(&sv->ms[0], sv->ev[0], sv->ev[1]));
+    sv->t_setup = false;
+  }
+  if (sv->t_setup_dl) {
+    VES3D_CK(cudaEventSynchronize(sv->ev[11]));
+    VES3D_CK(cudaEventElapsedTime(&sv->dl_ms, sv->ev[10], sv->ev[11]));
+    sv->t_setup_dl = false;
+  }
+  if (sv->check_tc) {
+    sv->check_tc = false;
+    if (tc_build_error(true)) {
+      sv->sl_valid = false;
+      set_error("self-matrix build on the tensor cores: a bounded wait of the kernel ran out");
+      return VES3D_ERR_CUDA;
+    }
+  }
+  return VES3D_OK;
+}
 
 // The self matrices of every vesicle: the single layer (SL), or with dl the double layer (DL).
-int run_setup(ves3d_sv* sv, bool dl) {
+// wait: until they are built (else the caller's collect_times takes the build's time and errors).
+int run_setup(ves3d_sv* sv, bool dl, bool wait) {
   NvtxRange nvtx(dl ? "ves3d build dl" : "ves3d build");
   const DevTables& T = sv->tab->d;
   const int p0 = sv->p, p1 = sv->pup, nc = ncoef_(p0), ng = ngrid_(p0), M1 = ngrid_(p1);
@@ -528,7 +568,7 @@ int run_setup(ves3d_sv* sv, bool dl) {
     set_error("internal: self-matrix build without its buffers");
     return VES3D_ERR_STATE;
   }
-  VES3D_CK(cudaEventRecord(sv->ev[0], st));
+  VES3D_CK(cudaEventRecord(sv->ev[dl ? 10 : 0], st));
   for (long v0 = 0; v0 < sv->nves; v0 += sv->chunk) {
     const long nb = std::min(sv->chunk, sv->nves - v0);
     const long nrot = nb * npr;
@@ -563,20 +603,15 @@ int run_setup(ves3d_sv* sv, bool dl) {
     (void)ng;
     (void)M1;
   }
-  VES3D_CK(cudaEventRecord(sv->ev[1], st));
-  VES3D_CK(cudaEventSynchronize(sv->ev[1]));
-  VES3D_CK(cudaEventElapsedTime(dl ? &sv->dl_ms : &sv->ms[0], sv->ev[0], sv->ev[1]));
-  if (tc && tc_build_error(true)) {
-    set_error("self-matrix build on the tensor cores: a bounded wait of the kernel ran out");
-    return VES3D_ERR_CUDA;
-  }
+  VES3D_CK(cudaEventRecord(sv->ev[dl ? 11 : 1], st));
   if (dl) {
-    sv->dl_valid = true;
+    sv->dl_valid = sv->t_setup_dl = true;
   } else {
-    sv->sl_valid = true;
+    sv->sl_valid = sv->t_setup = true;
     sv->sl_tc = tc || f32post;
+    sv->check_tc = tc;
   }
-  return VES3D_OK;
+  return wait ? collect_times(sv) : VES3D_OK;
 }
 
 // Self part of an evaluation: Vself = SHC2Grid(Grid2SHC(F) . SL) and the weighted far-field
@@ -660,11 +695,11 @@ int fork_far(ves3d_sv* sv, int* nseg, cudaEvent_t ev_far0, cudaEvent_t ev_far1, 
 // The self-matrix build on the high-priority stream (after everything queued on the
 // context's stream), the context's stream waiting for it.
 int run_setup_hi(ves3d_sv* sv) {
-  if (!sv->overlap) return run_setup(sv);
+  if (!sv->overlap) return run_setup(sv, false, /*wait=*/false);
   VES3D_CK(cudaStreamWaitEvent(sv->hi, sv->ev_fork, 0));
   cudaStream_t saved = sv->stream;
   sv->stream = sv->hi;
-  const int s = run_setup(sv);
+  const int s = run_setup(sv, false, /*wait=*/false);
   sv->stream = saved;
   if (s) return s;
   VES3D_CK(cudaEventRecord(sv->ev_built, sv->hi));
@@ -691,8 +726,8 @@ int run_eval_body(ves3d_sv* sv, bool dl) {
 
 // One evaluation; dl adds the double layer of the density G (the operator's own
 // evaluation when a double-layer density is set; the implicit step applies the single
-// layer alone).
-int run_eval(ves3d_sv* sv, bool dl) {
+// layer alone). wait: until it is done (else it is queued, its times left to collect_times).
+int run_eval(ves3d_sv* sv, bool dl, bool wait = true) {
   cudaStream_t st = sv->stream;
   int s, nseg = 0;
   if (!sv->have_src || !sv->have_den) {
@@ -708,18 +743,16 @@ int run_eval(ves3d_sv* sv, bool dl) {
   }
   if ((s = fork_far(sv, &nseg, sv->ev[4], sv->ev[5], dl))) return s;
   if (!sv->sl_valid && (s = run_setup_hi(sv))) return s;
-  if (dl && !sv->dl_valid && (s = run_setup(sv, true))) return s;
+  if (dl && !sv->dl_valid && (s = run_setup(sv, true, /*wait=*/false))) return s;
   VES3D_CK(cudaEventRecord(sv->ev[2], st));
   if ((s = run_self_apply(sv, dl))) return s;
   VES3D_CK(cudaEventRecord(sv->ev[3], st));
   if ((s = join_far(sv, nseg, dl))) return s;
   VES3D_CK(cudaEventRecord(sv->ev[6], st));
-  VES3D_CK(cudaEventSynchronize(sv->ev[6]));
-  VES3D_CK(cudaEventElapsedTime(&sv->ms[1], sv->ev[2], sv->ev[3]));
-  VES3D_CK(cudaEventElapsedTime(&sv->ms[2], sv->ev[4], sv->ev[5]));
-  VES3D_CK(cudaEventElapsedTime(&sv->ms[3], sv->ev[2], sv->ev[6]));
-  sv->far_dl_ms = 0;
-  if (dl) VES3D_CK(cudaEventElapsedTime(&sv->far_dl_ms, sv->ev[8], sv->ev[9]));
+  sv->t_eval = true;
+  sv->t_eval_dl = dl;
+  // (the tensor-core build's result is checked before it is used further)
+  if ((wait || sv->check_tc) && (s = collect_times(sv))) return s;
   sv->parts_valid = true;
   return VES3D_OK;
 }
@@ -896,6 +929,7 @@ int ves3d_sv_create(int sh_order, int sh_order_up, int precision, int device, ve
   VES3D_CK(cudaEventCreateWithFlags(&sv->ev_join, cudaEventDisableTiming));
   VES3D_CK(cudaEventCreateWithFlags(&sv->ev_built, cudaEventDisableTiming));
   for (auto& ev : sv->ev) VES3D_CK(cudaEventCreate(&ev));
+  VES3D_CK(cudaEventCreateWithFlags(&sv->ev_copied, cudaEventDisableTiming));
   sv->tab.reset(new TablesOwner());
   build_tables(sh_order, sh_order_up, sv->tab->h);
   int s = sv->tab->upload(sv->stream);
@@ -931,6 +965,7 @@ int ves3d_sv_set_src_coord(ves3d_sv* sv, const double* S, long n_ves, int is_dev
   const int p0 = sv->p, ng = ngrid_(p0);
   const DevTables& T = sv->tab->d;
   if ((s = copy_in(sv->X, S, (size_t)n_ves * 3 * ng, is_device, sv->stream))) return s;
+  VES3D_CK(cudaEventRecord(sv->ev_copied, sv->stream));
   if (sv->off_nves != n_ves) {  // point offsets of the vesicles, uploaded when the count changes
     std::vector<long> off(n_ves + 1);
     for (long v = 0; v <= n_ves; v++) off[v] = v * ng;
@@ -946,7 +981,7 @@ int ves3d_sv_set_src_coord(ves3d_sv* sv, const double* S, long n_ves, int is_dev
   if ((s = launch_far_sources(sv->X, nullptr, sv->Xt, sv->Xp, n_ves, p0, T.smooth_w0, sv->area, sv->pos, nullptr,
                               sv->stream)))
     return s;
-  VES3D_CK(cudaStreamSynchronize(sv->stream));
+  VES3D_CK(cudaEventSynchronize(sv->ev_copied));  // S has been read
   sv->have_src = true;
   sv->have_den = false;
   sv->have_dl = false;  // densities belong to the surfaces they were set for
@@ -1297,12 +1332,16 @@ int ves3d_sv_get_parts(ves3d_sv* sv, double* vel_self, double* vel_far, int is_d
 
 int ves3d_sv_stage_times(ves3d_sv* sv, float* ms) {
   VES3D_ARG(sv != nullptr && ms != nullptr, "null argument");
+  const int s = collect_times(sv);
+  if (s) return s;
   for (int i = 0; i < 4; i++) ms[i] = sv->ms[i];
   return VES3D_OK;
 }
 
 int ves3d_sv_far_dl_time(ves3d_sv* sv, float* ms) {
   VES3D_ARG(sv != nullptr && ms != nullptr, "null argument");
+  const int s = collect_times(sv);
+  if (s) return s;
   *ms = sv->far_dl_ms;
   return VES3D_OK;
 }
@@ -1876,7 +1915,7 @@ int stokes_apply(ves3d_sv* sv, const double* f, double* out, bool dl = false) {
   VES3D_CK(cudaMemcpyAsync(sv->F, f, n * sizeof(double), cudaMemcpyDeviceToDevice, sv->stream));
   sv->have_den = true;
   if (dl) sv->have_dl = false;
-  if ((s = run_eval(sv, dl))) return s;
+  if ((s = run_eval(sv, dl, /*wait=*/false))) return s;
   VES3D_CK(cudaMemcpyAsync(out, sv->V, n * sizeof(double), cudaMemcpyDeviceToDevice, sv->stream));
   return VES3D_OK;
 }
@@ -2696,22 +2735,16 @@ int ves3d_sv_surface_op(ves3d_sv* sv, int op, const double* in, double* out, int
     default: VES3D_ARG(false, "unknown surface op");
   }
   VES3D_ARG(nin == 0 || in != nullptr, "in is null");
-  double *din = nullptr, *dout = nullptr;
-  int st = VES3D_OK;
-  if (nin && (st = dalloc(&din, nin))) return st;
-  if ((st = dalloc(&dout, nout))) {
-    dfree(din);
-    return st;
-  }
-  if (nin) st = copy_in(din, in, nin, is_device, sv->stream);
+  // the operand and the result go through two vectors of the work space that the grid-space
+  // operations leave alone
   ImplicitWork iw;
-  if (!st) st = implicit_work(sv, iw);
+  int st = implicit_work(sv, iw);
+  if (st) return st;
+  double *din = iw.g1, *dout = iw.g2;
+  if (nin) st = copy_in(din, in, nin, is_device, sv->stream);
   if (!st) {
     switch (op) {
-      case VES3D_OP_GEOMETRY:
-        st = cuda_status(cudaMemcpyAsync(dout, sv->geo, nout * sizeof(double), cudaMemcpyDeviceToDevice, sv->stream),
-                         "copy", __FILE__, __LINE__);
-        break;
+      case VES3D_OP_GEOMETRY: dout = sv->geo; break;
       case VES3D_OP_GRAD: st = op_grad(sv, din, dout); break;
       case VES3D_OP_DIV: st = op_div(sv, din, dout, 1.0); break;
       case VES3D_OP_LIN_MEANCURV: st = op_linH(sv, din, dout); break;
@@ -2736,8 +2769,6 @@ int ves3d_sv_surface_op(ves3d_sv* sv, int op, const double* in, double* out, int
   }
   if (!st) st = copy_out(out, dout, nout, is_device, sv->stream);
   cudaStreamSynchronize(sv->stream);
-  dfree(din);
-  dfree(dout);
   return st;
 }
 
@@ -3321,16 +3352,18 @@ int ves3d_svp_set_viscosity_contrast(ves3d_svp* g, const double* lambda, long n)
   return VES3D_OK;
 }
 
-int ves3d_svp_setup(ves3d_svp* g) {
+static int svp_setup(ves3d_svp* g, bool wait) {
   VES3D_ARG(g != nullptr, "null context");
   VES3D_ARG(!g->grp.empty(), "set_src_coord first");
   for (ves3d_sv* sv : g->grp) {
     int s;
-    if (!sv->sl_valid && (s = run_setup(sv))) return s;
-    if (g->have_dl && !sv->dl_valid && (s = run_setup(sv, true))) return s;
+    if (!sv->sl_valid && (s = run_setup(sv, false, wait))) return s;
+    if (g->have_dl && !sv->dl_valid && (s = run_setup(sv, true, wait))) return s;
   }
   return VES3D_OK;
 }
+
+int ves3d_svp_setup(ves3d_svp* g) { return svp_setup(g, true); }
 
 // every group's self part (with dl, of both layers: the DL matrices are built on first use)
 static int svp_self_parts(ves3d_svp* g, bool dl) {
@@ -3423,13 +3456,15 @@ int ves3d_svp_eval(ves3d_svp* g, double* vel, int is_device) {
   VES3D_CK(cudaSetDevice(g->device));
   int s;
   VES3D_CK(cudaEventRecord(g->ev[0], g->stream));
-  if ((s = ves3d_svp_setup(g))) return s;
+  if ((s = svp_setup(g, /*wait=*/false))) return s;
   VES3D_CK(cudaEventRecord(g->ev[1], g->stream));
   if ((s = svp_self_parts(g, g->have_dl))) return s;
   VES3D_CK(cudaEventRecord(g->ev[2], g->stream));
   if ((s = svp_far(g, g->have_dl))) return s;
   VES3D_CK(cudaEventRecord(g->ev[3], g->stream));
   VES3D_CK(cudaEventSynchronize(g->ev[3]));
+  for (ves3d_sv* sv : g->grp)
+    if ((s = collect_times(sv))) return s;
   VES3D_CK(cudaEventElapsedTime(&g->ms[0], g->ev[0], g->ev[1]));
   VES3D_CK(cudaEventElapsedTime(&g->ms[1], g->ev[1], g->ev[2]));
   VES3D_CK(cudaEventElapsedTime(&g->ms[2], g->ev[2], g->ev[3]));
