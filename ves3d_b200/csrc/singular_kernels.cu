@@ -333,17 +333,24 @@ __global__ void __launch_bounds__(256) k_rotate_transpose_scatter(const double* 
 // The rotate-transpose per (degree, order) item, in the arithmetic type TV: one CTA per
 // (latitude rotation t, vesicle v); for each pole and symmetric component the P longitude
 // rows of C are staged in degree-major order, then each thread takes one item (degree n,
-// order m): the coefficient of cos(m phi) and its sin(m phi) partner (one coefficient for
-// m = 0 and m = P), and forms for all P rows the rotation back
+// order m) -- the coefficient of cos(m phi) and its sin(m phi) partner (one coefficient for
+// m = 0 and m = P) -- and JH of the P rows, and forms the rotation back
 //     B[row][po + b] = sum_k A[row][po + k] Mr_{t,n}[b][k]
-// at its two positions b, then the inverse longitude phase of the pair in registers and
-// the P consecutive grid values of each coefficient as 16-byte vector stores into the
-// self-matrix grid SL3, laid out as the other forms'. A thread's rows share the staged
-// inputs (broadcast to the lanes of its degree) and its two rotation rows: 18 shared loads
-// per 32 FMAs at p = 16. TV = float in the mixed form (C is FP32 after the tensor-core
-// build, FP64 after the FP64 ring and rounded when staged; the FP32 grid goes to the FP32
-// Grid2SHC); TV = double in the FP64 form at p = 16 (the DMMA kernel below keeps the
-// other orders up to 16).
+// at its two positions b, then the inverse longitude phase of the pair in registers. The
+// values pass through shared memory (in place of the rows) to the self-matrix grid SL3, laid
+// out as the other forms', as whole rows of P consecutive grid values. A thread's rows share
+// the staged inputs (broadcast to the lanes of its degree) and its two rotation rows.
+// TV = float in the mixed form (C is FP32 after the tensor-core build, FP64 after the FP64 ring
+// and rounded when staged; the FP32 grid goes to the FP32 Grid2SHC); TV = double in the FP64
+// form (the DMMA kernel below keeps the odd orders).
+// Its data (C read and SL3 written once) would take a fifth of its time: what bounds it is
+// latency, with few warps per SM beside the tables in shared memory. So the rows of an item are
+// split over H threads, the next plane's inputs are sent for while this one is formed (to L2: in
+// registers they spill), and the output leaves in 16-byte stores of neighbouring lanes. A thread per
+// item that stored its own rows (32 lines per instruction) and now:
+//   FP64, p = 16, 512 / 64 vesicles  5.80 -> 3.86 ms / 775 -> 533 us
+//   FP32 of FP64, p = 24, 64         5.09 -> 2.30 ms
+//   FP32, p = 16, 512                2.84 -> 2.50 ms
 // The 16-byte vector of 16 / sizeof(T) values starting at o[i] (destinations 16-byte aligned).
 __device__ __forceinline__ float4 vec16(const float* o, int i) { return make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]); }
 __device__ __forceinline__ double2 vec16(const double* o, int i) { return make_double2(o[i], o[i + 1]); }
@@ -351,29 +358,43 @@ __device__ __forceinline__ double2 vec16(const double* o, int i) { return make_d
 template <int P, typename TV>
 struct RtItemCfg {
   static constexpr int NI = (P + 1) * (P + 2) / 2;  // items (n, m <= n), degree-major: n (n + 1) / 2 + m
-  static constexpr int NT = (NI + 31) / 32 * 32;   // one item per thread
+  static constexpr int NTI = (NI + 31) / 32 * 32;
+  static constexpr int W = 16 / sizeof(TV);  // values per 16-byte vector
+  // threads per item: whole vectors of rows each
+  static constexpr int H = P % (2 * W) == 0 ? 2 : P % (3 * W) == 0 ? 3 : 1;
+  static constexpr int JH = P / H, NT = H * NTI;
   // CTAs per SM the registers are sized for (shared memory allows 4 in FP32, 2 in FP64 at p = 16)
-  static constexpr int MINB = P == 16 ? (sizeof(TV) == 4 ? 4 : 2) : 1;
+  static constexpr int MINB = P <= 8 || (P <= 16 && sizeof(TV) == 4) ? 4 : P <= 12 ? 3 : P <= 16 ? 2 : 1;
+  // output row stride: 16-byte stores of eight neighbouring items fall on distinct banks
+  static constexpr int LDO = P + (sizeof(TV) == 4 ? (P % 8 == 4 ? 0 : 4) : (P % 4 == 2 ? 0 : 2));
+  // values of the rows [P][nc + 1], or of the outputs [2 NI][LDO] that take their place
+  static constexpr int SZA = (P * (P * (P + 2) + 1) > 2 * NI * LDO ? P * (P * (P + 2) + 1) : 2 * NI * LDO) + W - 1 & ~(W - 1);
+  static_assert(P % W == 0 && JH % W == 0, "rows of whole vectors");
 };
 
 template <int P, typename TC, typename TV>
 __global__ void __launch_bounds__(RtItemCfg<P, TV>::NT, RtItemCfg<P, TV>::MINB)
     k_rotate_transpose_item(const TC* __restrict__ C, int mr_per_t, DevTables T, TV* __restrict__ SL3) {
+  using Cf = RtItemCfg<P, TV>;
   constexpr int nc = P * (P + 2), ng = 2 * P * (P + 1), lda = nc + 1;
-  constexpr int NI = RtItemCfg<P, TV>::NI, NT = RtItemCfg<P, TV>::NT;
+  constexpr int NI = Cf::NI, NT = Cf::NT, JH = Cf::JH, W = Cf::W, LDO = Cf::LDO;
+  constexpr int LINE = 128 / sizeof(TC);
+  using V = decltype(vec16((const TV*)nullptr, 0));
   extern __shared__ __align__(16) unsigned char smraw[];
-  TV* sA = reinterpret_cast<TV*>(smraw);  // [P rows][lda], degree-major
-  TV* sM = sA + P * lda;                  // blocks of degree n at sMo[n], rows of bn | 1
+  TV* sA = reinterpret_cast<TV*>(smraw);  // [P rows][lda], degree-major, then the outputs [2][NI][LDO]
+  TV* sM = sA + Cf::SZA;                  // blocks of degree n at sMo[n], rows of bn | 1
   const int msz = mr_per_t + (P + 1) * 2 * P;  // (upper bound of the padded size)
   TV* sCs = sM + msz;                     // cos_tab [2P]
   TV* sSn = sCs + 2 * P;                  // sin_tab [2P]
   int* sMo = reinterpret_cast<int*>(sSn + 2 * P);                        // [P + 2] padded block offsets
   unsigned short* sDm = reinterpret_cast<unsigned short*>(sMo + P + 2);  // degree-major position [nc]
-  short* sI0 = reinterpret_cast<short*>(sDm + nc);                       // cos (or single) coefficient [NI]
+  unsigned short* sOr = sDm + nc;                                        // output row of a coefficient [nc]
+  short* sI0 = reinterpret_cast<short*>(sOr + nc);                       // cos (or single) coefficient [NI]
   short* sI1 = sI0 + NI;                                                 // its sin partner or -1 [NI]
   const int t = blockIdx.x;
   const long v = blockIdx.y;
   const int tid = threadIdx.x;
+  const TC* Cv = C + (v * (P + 1) + t) * P * 12 * (long)nc;  // [j][pole][comp][c]
   if (tid == 0) {
     int o = 0;
     for (int n = 0; n <= P; n++) {
@@ -391,13 +412,12 @@ __global__ void __launch_bounds__(RtItemCfg<P, TV>::NT, RtItemCfg<P, TV>::MINB)
   __syncthreads();
   for (int c = tid; c < nc; c += NT) {
     const int n = __ldg(T.n_of_coef + c), item = n * (n + 1) / 2 + __ldg(T.m_of_coef + c);
+    const bool sine = __ldg(T.is_sin + c);
     sDm[c] = (unsigned short)(__ldg(T.perm_off + n) + __ldg(T.pos_in_block + c));
-    if (__ldg(T.is_sin + c))
-      sI1[item] = (short)c;
-    else
-      sI0[item] = (short)c;
+    sOr[c] = (unsigned short)(item + (sine ? NI : 0));
+    (sine ? sI1 : sI0)[item] = (short)c;
   }
-  // the rotation blocks of this t, FP32, rows padded to bn | 1
+  // the rotation blocks of this t, rows padded to bn | 1
   for (int n = 0; n <= P; n++) {
     const int bn = __ldg(T.perm_off + n + 1) - __ldg(T.perm_off + n);
     const double* M = T.mr + __ldg(T.mr_off + t * (P + 1) + n);
@@ -407,50 +427,50 @@ __global__ void __launch_bounds__(RtItemCfg<P, TV>::NT, RtItemCfg<P, TV>::MINB)
     }
   }
   __syncthreads();
-  // this thread's item
+  // this thread's item and first row
+  const int item = tid % Cf::NTI, j0 = tid / Cf::NTI * JH;
   int n = 0;
-  while ((n + 1) * (n + 2) / 2 <= tid && n < P) n++;
-  const bool active = tid < NI && sI0[tid] >= 0;  // (every (n, m <= n) has its cos coefficient)
-  const int m = active ? tid - n * (n + 1) / 2 : 0;
-  const int c0 = active ? sI0[tid] : 0, c1 = active ? sI1[tid] : -1;
+  while ((n + 1) * (n + 2) / 2 <= item && n < P) n++;
+  const bool active = item < NI && sI0[item] >= 0;  // (every (n, m <= n) has its cos coefficient)
+  const int m = active ? item - n * (n + 1) / 2 : 0;
+  const int c0 = active ? sI0[item] : 0, c1 = active ? sI1[item] : -1;
   const int po = __ldg(T.perm_off + n), bn = __ldg(T.perm_off + n + 1) - po;
   const TV* M0 = active ? sM + sMo[n] + (sDm[c0] - po) * (bn | 1) : sM;
   const TV* M1 = c1 >= 0 ? sM + sMo[n] + (sDm[c1] - po) * (bn | 1) : M0;
   for (int pc = blockIdx.z; pc < 12; pc += gridDim.z) {
     const int pole = pc / 6, comp = pc - 6 * pole;
     const int grid0 = pole == 0 ? t * 2 * P : (P - t) * 2 * P + P;
-    {
-      __syncthreads();
-      // stage: A[j][dm(c)] = C[v][t][j][pole][comp][c], eight loads in flight per thread
-      for (int i0 = tid; i0 < P * nc; i0 += NT * 8) {
-        TV val[8];
+    // stage A[j][dm(c)], eight loads in flight per thread
+#pragma unroll 1
+    for (int i0 = tid; i0 < P * nc; i0 += NT * 8) {
+      TC val[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int i = i0 + u * NT;
-          if (i < P * nc) {
-            const int j = i / nc, c = i - j * nc;
-            val[u] = (TV)C[((((v * (P + 1) + t) * P + j) * 2 + pole) * 6 + comp) * (long)nc + c];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int i = i0 + u * NT;
-          if (i < P * nc) {
-            const int j = i / nc, c = i - j * nc;
-            sA[j * lda + sDm[c]] = val[u];
-          }
-        }
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + u * NT, j = i / nc;
+        if (i < P * nc) val[u] = Cv[((long)j * 12 + pc) * nc + (i - j * nc)];
       }
-      __syncthreads();
-      if (!active) continue;
-      TV acc0[P], acc1[P];
 #pragma unroll
-      for (int j = 0; j < P; j++) acc0[j] = acc1[j] = TV(0);
-      const TV* a = sA + po;
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + u * NT, j = i / nc;
+        if (i < P * nc) sA[j * lda + sDm[i - j * nc]] = (TV)val[u];
+      }
+    }
+    __syncthreads();
+    // the next plane on its way to L2
+    if (pc + gridDim.z < 12)
+      for (int i = tid; i < P * ((nc + LINE - 1) / LINE); i += NT) {
+        const int j = i % P, l = i / P;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(Cv + ((long)j * 12 + pc + gridDim.z) * nc + min(l * LINE, nc - 1)));
+      }
+    TV acc0[JH], acc1[JH];
+#pragma unroll
+    for (int j = 0; j < JH; j++) acc0[j] = acc1[j] = TV(0);
+    if (active) {
+      const TV* a = sA + j0 * lda + po;
       for (int k = 0; k < bn; k++) {
         const TV m0 = M0[k], m1 = M1[k];
 #pragma unroll
-        for (int j = 0; j < P; j++) {
+        for (int j = 0; j < JH; j++) {
           const TV x = a[j * lda + k];
           acc0[j] = fma(x, m0, acc0[j]);
           acc1[j] = fma(x, m1, acc1[j]);
@@ -459,39 +479,44 @@ __global__ void __launch_bounds__(RtItemCfg<P, TV>::NT, RtItemCfg<P, TV>::MINB)
       // inverse longitude phase of the pair: cos row c0, sin row c1
       if (c1 >= 0) {
 #pragma unroll
-        for (int j = 0; j < P; j++) {
-          const int q = (m * j) % (2 * P);
+        for (int j = 0; j < JH; j++) {
+          const int q = (m * (j0 + j)) % (2 * P);
           const TV cs = sCs[q], sn = sSn[q];
           const TV x0 = acc0[j], x1 = acc1[j];
           acc0[j] = fma(-x1, sn, x0 * cs);
           acc1[j] = fma(x0, sn, x1 * cs);
         }
       }
-      // symmetric component -> (c_in, c_out): (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)
-      const int cin = comp < 3 ? 0 : (comp < 5 ? 1 : 2), cout = comp < 3 ? comp : (comp < 5 ? comp - 2 : 2);
-      auto put = [&](int c, const TV* o) {
-        TV* d0 = SL3 + (((v * 3 + cin) * nc + c) * 3 + cout) * (long)ng + grid0;
-        TV* d1 = SL3 + (((v * 3 + cout) * nc + c) * 3 + cin) * (long)ng + grid0;
-        using V = decltype(vec16(o, 0));
-        constexpr int W = 16 / sizeof(TV);
-#pragma unroll
-        for (int q = 0; q < P / W; q++) {
-          const V w = vec16(o, W * q);
-          reinterpret_cast<V*>(d0)[q] = w;
-          if (cin != cout) reinterpret_cast<V*>(d1)[q] = w;
-        }
-      };
-      put(c0, acc0);
-      if (c1 >= 0) put(c1, acc1);
     }
+    __syncthreads();
+    if (active) {
+      V* o = reinterpret_cast<V*>(sA + item * LDO + j0);
+#pragma unroll
+      for (int q = 0; q < JH / W; q++) {
+        o[q] = vec16(acc0, W * q);
+        if (c1 >= 0) o[q + NI * LDO / W] = vec16(acc1, W * q);
+      }
+    }
+    __syncthreads();
+    // symmetric component -> (c_in, c_out): (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)
+    const int cin = comp < 3 ? 0 : (comp < 5 ? 1 : 2), cout = comp < 3 ? comp : (comp < 5 ? comp - 2 : 2);
+    TV* d0 = SL3 + ((v * 3 + cin) * nc * 3 + cout) * (long)ng + grid0;
+    TV* d1 = SL3 + ((v * 3 + cout) * nc * 3 + cin) * (long)ng + grid0;
+#pragma unroll 4
+    for (int i = tid; i < nc * (P / W); i += NT) {
+      const int c = i / (P / W), q = i - c * (P / W);
+      const V w = reinterpret_cast<const V*>(sA + sOr[c] * LDO)[q];
+      reinterpret_cast<V*>(d0 + (long)c * 3 * ng)[q] = w;
+      if (cin != cout) reinterpret_cast<V*>(d1 + (long)c * 3 * ng)[q] = w;
+    }
+    __syncthreads();
   }
 }
 
-template <typename TV>
-static size_t rt_item_smem(int p0, int mpt) {
-  const int nc = p0 * (p0 + 2), lda = nc + 1, ni = (p0 + 1) * (p0 + 2) / 2;
-  const size_t fl = (size_t)p0 * lda + mpt + (size_t)(p0 + 1) * 2 * p0 + 4 * p0;
-  return fl * sizeof(TV) + (size_t)(p0 + 2) * sizeof(int) + (size_t)nc * 2 + (size_t)ni * 4 + 16;
+template <int P, typename TV>
+static size_t rt_item_smem(int mpt) {
+  const size_t fl = (size_t)RtItemCfg<P, TV>::SZA + mpt + (size_t)(P + 1) * 2 * P + 4 * P;
+  return fl * sizeof(TV) + (size_t)(P + 2) * sizeof(int) + (size_t)P * (P + 2) * 4 + (size_t)RtItemCfg<P, TV>::NI * 4 + 16;
 }
 
 template <int P, typename TC, typename TV = float>
@@ -502,7 +527,7 @@ static int launch_rt_item(const TC* C, long nv, const DevTables& T, TV* SL3, cud
   int planes = 1;
   while (planes < 12 && (P + 1) * nv * planes < 4 * 148) planes = planes < 4 ? planes + 1 : planes == 4 ? 6 : 12;
   dim3 grid(P + 1, (unsigned)nv, (unsigned)planes);
-  const size_t smem = rt_item_smem<TV>(P, mpt);  // about 48 KB at p = 16 (four CTAs per SM), 149 KB at p = 24
+  const size_t smem = rt_item_smem<P, TV>(mpt);  // FP32: 53 KB at p = 16 (four CTAs per SM), 163 KB at p = 24
   VES3D_CK(cudaFuncSetAttribute(k_rotate_transpose_item<P, TC, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)smem));
   k_rotate_transpose_item<P, TC, TV><<<grid, RtItemCfg<P, TV>::NT, smem, st>>>(C, mpt, T, SL3);
@@ -697,7 +722,7 @@ __global__ void __launch_bounds__(256, 2) k_rotate_transpose_tc(const double* __
 int launch_rotate_transpose_scatter(const double* C, long nv, const DevTables& T, double* SL3, cudaStream_t st) {
   if (nv <= 0) return VES3D_OK;
   const int p0 = T.p0, nc = ncoef_(p0);
-  // the per-item kernel in FP64 at its even orders (p = 16: 5.8 ms per 512-vesicle build against
+  // the per-item kernel in FP64 at its even orders (p = 16: 3.9 ms per 512-vesicle build against
   // 9.5 ms for the DMMA form below, which keeps the odd orders; p = 12, 8 vesicles: 51 against 128 us;
   // whole builds of 27 vesicles at p = 4 38 against 54 us, p = 20 4.9 against 7.6 ms)
   if (!tc_rotate_disabled()) switch (p0) {
