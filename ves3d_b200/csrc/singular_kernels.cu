@@ -10,88 +10,101 @@
 
 namespace ves3d {
 
-// One CTA per (vesicle v, latitude rotation t); loops over the p0 longitude phases j, JB
-// of them at a time (4, or fewer where the staging would not fit: p = 24).
+// Most threads (coefficients) a CTA takes: the rotation blocks of larger orders outgrow shared memory.
+constexpr int kRotAllMax = 768;
+
+// CTAs (vesicle v, latitude rotation t, part of the p0 longitude phases j), JB phases at a time (4,
+// or fewer where the staging would not fit: p = 24).
 // out[c'] = sum_b (P_j s)[perm_n[b]] * Mr[t][n][b][pos(c')],   n = degree(c').
-// The blocks Mr[t][.] (mr_per_t doubles, contiguous for one t) are staged in shared memory.
-// Outputs are formed in degree-major order (a warp's lanes share a degree: one loop length,
-// broadcast inputs, consecutive block columns) and each thread forms its coefficient for
-// JB longitudes at once, reusing every block element.
+// A thread per coefficient: it keeps the coefficient and its partner in registers, writes their JB
+// phases to shared memory in degree-major order, and forms one degree-major output of the three
+// components and JB phases (a warp's lanes share a degree: one loop length, broadcast inputs in
+// 16-byte loads, consecutive block columns), so a block element is loaded once per 3 JB
+// multiply-adds. The outputs return to their order in shared memory and leave as one contiguous run.
+// The data (R written once) would take a third of its time; bound by the shared-memory loads and the
+// barriers around them. With four multiply-adds per block element, one component a pass, and outputs
+// stored in degree-major order (8 bytes per line) it took
+//   p = 16, 512 / 64 vesicles  1.71 ms / 240 us, now 1.10 ms / 154 us
+//   p = 24, 64 vesicles        2.59 ms, now 0.86 ms
 template <int JB>
-__global__ void __launch_bounds__(256) k_rotate_all(const double* __restrict__ S, int p0, int mr_per_t, DevTables T,
-                                                    double* __restrict__ R) {
-  constexpr int kRaJ = JB;
-  extern __shared__ double sm[];
+__global__ void __launch_bounds__(kRotAllMax) k_rotate_all(const double* __restrict__ S, int p0, int mr_per_t,
+                                                           DevTables T, double* __restrict__ R) {
+  constexpr int ND = 3 * JB, LDB = JB == 4 ? 14 : ND + (JB & 1);  // (row stride: even, off the multiples of 16)
+  extern __shared__ __align__(16) double sm[];
   const int nc = p0 * (p0 + 2);
-  double* sS = sm;
-  double* sB = sm + 3 * nc;                                        // [kRaJ][3 nc]
-  double* sM = sB + kRaJ * 3 * nc;
-  double* sCs = sM + mr_per_t;                                     // cos_tab [2 p0]
-  double* sSn = sCs + 2 * p0;                                      // sin_tab [2 p0]
-  int* sMo = reinterpret_cast<int*>(sSn + 2 * p0);                 // mr_off of (t, n) - base [p0 + 1]
-  int* sPo = sMo + (p0 + 1);                                       // perm_off [p0 + 2]
-  short* sPc = reinterpret_cast<short*>(sPo + (p0 + 2));           // partner [nc]
-  unsigned short* sPerm = reinterpret_cast<unsigned short*>(sPc + nc);  // perm [nc]
-  unsigned char* sMs = reinterpret_cast<unsigned char*>(sPerm + nc);    // m | (is_sin << 7) [nc]
-  unsigned char* sNd = sMs + nc;                                   // degree of degree-major position [nc]
+  double* sB = sm;                                  // phases [nc][LDB], then outputs [JB][3][nc]
+  double* sM = sB + (size_t)LDB * nc;               // blocks of t, rows b
+  double* sCs = sM + mr_per_t;                      // cos_tab [2 p0]
+  double* sSn = sCs + 2 * p0;                       // sin_tab [2 p0]
   const int t = blockIdx.x;
   const long v = blockIdx.y;
+  const int tid = threadIdx.x;
   const int mbase = __ldg(T.mr_off + t * (p0 + 1));
-  for (int i = threadIdx.x; i < 3 * nc; i += blockDim.x) sS[i] = S[v * 3 * nc + i];
-  for (int i = threadIdx.x; i < mr_per_t; i += blockDim.x) sM[i] = __ldg(T.mr + mbase + i);
-  for (int i = threadIdx.x; i < 2 * p0; i += blockDim.x) {
+  for (int i = tid; i < mr_per_t; i += blockDim.x) sM[i] = __ldg(T.mr + mbase + i);
+  for (int i = tid; i < 2 * p0; i += blockDim.x) {
     sCs[i] = __ldg(T.cos_tab + i);
     sSn[i] = __ldg(T.sin_tab + i);
   }
-  for (int i = threadIdx.x; i <= p0; i += blockDim.x) sMo[i] = __ldg(T.mr_off + t * (p0 + 1) + i) - mbase;
-  for (int i = threadIdx.x; i <= p0 + 1; i += blockDim.x) sPo[i] = __ldg(T.perm_off + i);
-  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-    sPc[c] = (short)__ldg(T.partner + c);
-    sPerm[c] = (unsigned short)__ldg(T.perm + c);
-    sMs[c] = (unsigned char)(__ldg(T.m_of_coef + c) | (__ldg(T.is_sin + c) ? 0x80 : 0));
-    const int n = __ldg(T.n_of_coef + c);
-    sNd[__ldg(T.perm_off + n) + __ldg(T.pos_in_block + c)] = (unsigned char)n;
+  // thread tid holds coefficient c = tid for the phases and degree-major position e = tid for the sums
+  const bool active = tid < nc;
+  const int c = active ? tid : 0;
+  const int pc = __ldg(T.partner + c), m = __ldg(T.m_of_coef + c), n = __ldg(T.n_of_coef + c);
+  const bool sine = __ldg(T.is_sin + c);
+  const int dm = __ldg(T.perm_off + n) + __ldg(T.pos_in_block + c);
+  double own[3], other[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    own[d] = S[(v * 3 + d) * nc + c];
+    other[d] = pc >= 0 ? S[(v * 3 + d) * nc + pc] : 0.0;
   }
-  __syncthreads();
-  for (int j0 = 0; j0 < p0; j0 += kRaJ) {
-    const int nj = min(kRaJ, p0 - j0);
-    for (int i = threadIdx.x; i < nj * 3 * nc; i += blockDim.x) {
-      const int jj = i / (3 * nc), r = i - jj * 3 * nc;
-      const int d = r / nc, c = r - d * nc;
-      const int pc = sPc[c];
-      double val;
-      if (pc < 0) {
-        val = sS[r];
-      } else {
-        const int ms = sMs[c];
-        const int q = ((ms & 0x7f) * (j0 + jj)) % (2 * p0);
+  const int ce = __ldg(T.perm + c), ne = __ldg(T.n_of_coef + ce);  // the output's coefficient and degree
+  const int po = __ldg(T.perm_off + ne), bn = __ldg(T.perm_off + ne + 1) - po;
+  const double* M = sM + __ldg(T.mr_off + t * (p0 + 1) + ne) - mbase + (c - po);
+  const int rounds = (p0 + JB - 1) / JB;
+  for (int r = blockIdx.z; r < rounds; r += gridDim.z) {
+    const int j0 = r * JB, nj = min(JB, p0 - j0);
+    __syncthreads();
+    if (active) {
+      int q = (m * j0) % (2 * p0);
+#pragma unroll
+      for (int jj = 0; jj < JB; jj++) {
         const double cs = sCs[q], sn = sSn[q];
-        val = (ms & 0x80) ? -sS[d * nc + pc] * sn + sS[r] * cs : sS[r] * cs + sS[d * nc + pc] * sn;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          double val = own[d];
+          if (pc >= 0) val = sine ? -other[d] * sn + own[d] * cs : own[d] * cs + other[d] * sn;
+          sB[dm * LDB + jj * 3 + d] = val;
+        }
+        q += m;
+        if (q >= 2 * p0) q -= 2 * p0;
       }
-      sB[jj * 3 * nc + r] = val;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * nc; i += blockDim.x) {
-      const int d = i / nc, e = i - d * nc;  // e: degree-major position of the output
-      const int n = sNd[e];
-      const int po = sPo[n], bn = sPo[n + 1] - po, bp = e - po;
-      const double* M = sM + sMo[n] + bp;
-      const double* b = sB + d * nc;
-      double acc[kRaJ];
+    double acc[ND];
 #pragma unroll
-      for (int q = 0; q < kRaJ; q++) acc[q] = 0.0;
+    for (int u = 0; u < ND; u++) acc[u] = 0.0;
+    if (active) {
+      const double* b = sB + po * LDB;
       for (int k = 0; k < bn; k++) {
-        const double m = M[k * bn];
-        const int src = sPerm[po + k];
+        const double w = M[k * bn];
+        double x[ND + (ND & 1)];
 #pragma unroll
-        for (int q = 0; q < kRaJ; q++) acc[q] = fma(b[q * 3 * nc + src], m, acc[q]);
+        for (int u = 0; u < (ND + 1) / 2; u++) {
+          const double2 y = reinterpret_cast<const double2*>(b + k * LDB)[u];
+          x[2 * u] = y.x;
+          x[2 * u + 1] = y.y;
+        }
+#pragma unroll
+        for (int u = 0; u < ND; u++) acc[u] = fma(x[u], w, acc[u]);
       }
-      const int c = sPerm[e];
-#pragma unroll
-      for (int q = 0; q < kRaJ; q++)
-        if (q < nj) R[(((v * (p0 + 1) + t) * p0 + j0 + q) * 3 + d) * (long)nc + c] = acc[q];
     }
     __syncthreads();
+    if (active)
+#pragma unroll
+      for (int u = 0; u < ND; u++) sB[u * nc + ce] = acc[u];
+    __syncthreads();
+    double* out = R + ((v * (p0 + 1) + t) * p0 + j0) * 3 * (long)nc;
+    for (int i = tid; i < nj * 3 * nc; i += blockDim.x) out[i] = sB[i];
   }
 }
 
@@ -145,25 +158,33 @@ int launch_rotate_all(const double* S, long nv, const DevTables& T, double* R, c
     set_error("rotation kernels support SH orders up to 127");
     return VES3D_ERR_ARG;
   }
-  auto smem_of = [&](int jb) {
-    return (((3 + 3 * (size_t)jb) * nc + mpt + 4 * p0) * sizeof(double) + (2 * p0 + 3) * sizeof(int) + nc * 4 + nc * 2 +
-            15) / 16 * 16;
-  };
-  dim3 grid(p0 + 1, (unsigned)nv);
   const size_t cap = 227 * 1024;
-  if (smem_of(4) <= cap) {
-    VES3D_CK(cudaFuncSetAttribute(k_rotate_all<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(4)));
-    k_rotate_all<4><<<grid, 256, smem_of(4), st>>>(S, p0, mpt, T, R);
-  } else if (smem_of(2) <= cap) {
-    VES3D_CK(cudaFuncSetAttribute(k_rotate_all<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(2)));
-    k_rotate_all<2><<<grid, 256, smem_of(2), st>>>(S, p0, mpt, T, R);
-  } else if (smem_of(1) <= cap) {
-    VES3D_CK(cudaFuncSetAttribute(k_rotate_all<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(1)));
-    k_rotate_all<1><<<grid, 256, smem_of(1), st>>>(S, p0, mpt, T, R);
-  } else {
+  int jb = 0;
+  size_t smem = 0;
+  for (int k : {4, 2, 1}) {
+    smem = ((size_t)(k == 4 ? 14 : 3 * k + (k & 1)) * nc + mpt + 4 * p0) * sizeof(double);
+    if (smem <= cap) {
+      jb = k;
+      break;
+    }
+  }
+  if (jb == 0 || nc > kRotAllMax) {
     set_error("RotateAll: the rotation blocks of p = %d do not fit in shared memory", p0);
     return VES3D_ERR_ARG;
   }
+  // few vesicles: the phases of a (vesicle, rotation) over several CTAs, up to two per SM
+  const int rounds = (p0 + jb - 1) / jb;
+  int parts = 1;
+  while (parts < rounds && (p0 + 1) * nv * parts < 2 * 148) parts++;
+  const dim3 grid(p0 + 1, (unsigned)nv, (unsigned)parts);
+  const int nt = ((int)nc + 31) / 32 * 32;
+  auto launch = [&](auto kernel) {
+    VES3D_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, nt, smem, st>>>(S, p0, mpt, T, R);
+    return (int)VES3D_OK;
+  };
+  const int s = jb == 4 ? launch(k_rotate_all<4>) : jb == 2 ? launch(k_rotate_all<2>) : launch(k_rotate_all<1>);
+  if (s) return s;
   VES3D_LAUNCHED();
   return VES3D_OK;
 }
