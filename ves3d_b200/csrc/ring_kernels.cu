@@ -22,7 +22,7 @@
 // phases and instruction fetch of the unrolled transforms. Self matrices of
 //   512 / 64 vesicles, p = 16:  32.8 -> 18.3 ms / 4.12 -> 2.28 ms  (before: dense, DMMA from shared memory)
 //   64 vesicles, p = 24:        32.4 -> 16.3 ms
-//   27 vesicles, p = 12:        1.29 -> 0.75 ms
+//   64 vesicles, p = 12:        1.29 -> 0.66 ms
 //   double layer, 48 at p = 16: 20 -> 1.72 ms  (before: a kernel per stage, intermediates in HBM)
 // Thread groups that take a pair each through all phases with their own barriers were slower
 // (2.91 ms for 64 vesicles), as were three or five parts per row (the code outgrows the cache).
@@ -71,11 +71,14 @@ __host__ __device__ constexpr int round16(int n, int r) { return n + ((r - n % 1
 // a CTA takes through the phases at a time (fewer where a large p_up leaves no room for them).
 // Threads are the items of the transposed Legendre sums; CTAs per SM what registers and shared memory
 // allow, several so that one CTA's barriers are another's work.
+// p = 12 in two CTAs of 192 threads and five pairs against three of 128 and three pairs (13 pairs in three
+// rounds for five): 64 vesicles 746 -> 660 us, 8 vesicles 111 -> 96 us, p_up = 40 2.72 -> 2.19 ms; p = 10
+// so was slower (310 -> 360 us).
 template <int P>
 struct RingShape {
-  static constexpr int NT = P <= 12 ? 128 : P <= 16 ? 192 : 384;
-  static constexpr int MINB = P <= 8 ? 4 : P <= 12 ? 3 : P <= 16 ? 2 : 1;
-  static constexpr int LPG = P == 12 ? 3 : P <= 16 ? 4 : 5;
+  static constexpr int NT = P <= 10 ? 128 : P <= 16 ? 192 : 384;
+  static constexpr int MINB = P <= 8 ? 4 : P <= 10 ? 3 : P <= 16 ? 2 : 1;
+  static constexpr int LPG = P <= 10 || P == 16 ? 4 : 5;
   static constexpr int QC = 4;  // coefficients of one transposed-Legendre item
   static constexpr int NP = 2;  // parts of a row in the DFT synthesis
   static_assert(legt_items(P, QC) <= NT, "one item per thread");
