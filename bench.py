@@ -692,7 +692,7 @@ def double_layer_measurement(X, f, p, local, stream, steps=3):
         ms = statistics.mean(far_dl)
         achieved = DL_FLOPS_PER_PAIR * pairs / (ms * 1e-3) / 1e12
         peak = fma_peak(prec == "fp64")
-        kernel = "k_far_dl_f64_flat" if prec == "fp64" else "k_far_dl_f32_flat"
+        kernel = "k_far_sym_f64" if prec == "fp64" else "k_far_dl_f32_flat"
         res[prec] = {"eval_ms": statistics.mean(evals), "far_dl_ms": ms, "first_eval_with_dl_build_s": first_s,
                      "far_dl_roofline": {"kernel": kernel, "bound": "fp64_pipe" if prec == "fp64" else "fp32_pipe",
                                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,

@@ -253,10 +253,11 @@ constexpr int kProjWarps = 4;
 // Projection of each near target on its vesicle and the on-surface values there: one group of G
 // lanes per (slot, target) pair, slot-major (most targets have one near vesicle, so the groups in
 // use are neighbours). The vesicle's coefficients and the recurrence tables are staged in shared
-// memory. 0.64 ms for 15,000 pairs at p = 12; what bounds it is the serial chain of up to 40 Gauss-Newton steps of p + 1 recurrence
+// memory. What bounds it is the serial chain of up to 40 Gauss-Newton steps of p + 1 recurrence
 // steps each: with the square roots and divisions of the recurrence in tables, 16 lanes per pair
-// at p <= 15 and every warp at it (one warp of a 128-thread CTA per pair, three waiting, and
-// the coefficients recomputed took 14.5 ms for 15,000 pairs at p = 12).
+// at p <= 15 and every warp at it, 15,000 pairs at p = 12 take 0.65 ms (one warp of a 128-thread CTA
+// per pair, three waiting, and the coefficients recomputed took 14.5 ms with the sums of
+// k_near_correct).
 template <int G>
 __global__ void __launch_bounds__(32 * kProjWarps) k_near_project(NearArgs A) {
   extern __shared__ double smn[];
