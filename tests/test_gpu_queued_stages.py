@@ -52,3 +52,25 @@ def test_surface_ops_after_queued_work():
             u, w = a.surface_op(op, arg), b.surface_op(op, arg)
             assert np.array_equal(u, w) and np.isfinite(u).all()
             assert np.array_equal(a.surface_op(op, arg), u)
+
+
+def test_another_stream_after_the_surfaces():
+    """A stream set after SetSrcCoord finds the surfaces' fields formed."""
+    import torch
+    p = 16
+    X, f = small_suspension(4, p, 21)
+    with StokesVelocity(p) as sv:
+        sv.SetSrcCoord(X)
+        sv.SetDensitySL(f)
+        ref = sv()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    dX, df = torch.from_numpy(X).cuda(), torch.from_numpy(f).cuda()
+    torch.cuda.synchronize()
+    with StokesVelocity(p) as sv:
+        for i in range(6):
+            sv.set_stream(streams[i % 2].cuda_stream)
+            sv.SetSrcCoord(dX)
+            sv.set_stream(streams[1 - i % 2].cuda_stream)
+            sv.SetDensitySL(df)
+            assert np.array_equal(sv(), ref)
+        sv.set_stream(None)

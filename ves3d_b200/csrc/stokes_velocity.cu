@@ -271,7 +271,7 @@ struct ves3d_sv {
   // [8, 9] far double layer, [10, 11] double-layer build. Their times are read when asked for, or
   // where the call waits for its result anyway (collect_times): the host queues a whole evaluation
   // without stopping between its stages.
-  cudaEvent_t ev[12] = {}, ev_copied = nullptr;
+  cudaEvent_t ev[12] = {}, ev_copied = nullptr, ev_src = nullptr;  // (ev_src: the surfaces' fields are formed)
   bool t_setup = false, t_setup_dl = false, t_eval = false, t_eval_dl = false, check_tc = false;
   float ms[4] = {0, 0, 0, 0};
   float far_dl_ms = 0;  // the far double layer's segment kernels in the last evaluation
@@ -295,6 +295,7 @@ struct ves3d_sv {
       if (e) cudaEventDestroy(e);
     tab.reset();
     if (ev_copied) cudaEventDestroy(ev_copied);
+    if (ev_src) cudaEventDestroy(ev_src);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_built) cudaEventDestroy(ev_built);
@@ -930,6 +931,7 @@ int ves3d_sv_create(int sh_order, int sh_order_up, int precision, int device, ve
   VES3D_CK(cudaEventCreateWithFlags(&sv->ev_built, cudaEventDisableTiming));
   for (auto& ev : sv->ev) VES3D_CK(cudaEventCreate(&ev));
   VES3D_CK(cudaEventCreateWithFlags(&sv->ev_copied, cudaEventDisableTiming));
+  VES3D_CK(cudaEventCreateWithFlags(&sv->ev_src, cudaEventDisableTiming));
   sv->tab.reset(new TablesOwner());
   build_tables(sh_order, sh_order_up, sv->tab->h);
   int s = sv->tab->upload(sv->stream);
@@ -949,6 +951,8 @@ int ves3d_sv_destroy(ves3d_sv* sv) {
 int ves3d_sv_set_stream(ves3d_sv* sv, void* stream) {
   int s = check_sv(sv);
   if (s) return s;
+  // what SetSrcCoord queued on the former stream comes before anything on the new one
+  VES3D_CK(cudaEventSynchronize(sv->ev_src));
   sv->stream = stream ? (cudaStream_t)stream : sv->own_stream;
   sv->drop_graph();
   return VES3D_OK;
@@ -981,6 +985,7 @@ int ves3d_sv_set_src_coord(ves3d_sv* sv, const double* S, long n_ves, int is_dev
   if ((s = launch_far_sources(sv->X, nullptr, sv->Xt, sv->Xp, n_ves, p0, T.smooth_w0, sv->area, sv->pos, nullptr,
                               sv->stream)))
     return s;
+  VES3D_CK(cudaEventRecord(sv->ev_src, sv->stream));
   VES3D_CK(cudaEventSynchronize(sv->ev_copied));  // S has been read
   sv->have_src = true;
   sv->have_den = false;
