@@ -154,14 +154,18 @@ __global__ void __launch_bounds__(128) k_near_find(const double* __restrict__ tr
 }
 
 // Recurrence tables of the normalised associated Legendre functions (near_tables): rows n = 0..p
-// of [3][32] (order m): a and b of P(m, n) = a x P(m, n - 1) - b P(m, n - 2), and c of the
-// derivative's P(m + 1, n) term; then [32] diagonal factors, P(m, m) = diag (-s)^m.
+// of [3][32] (order m): a and b of P(m, n) = x a P(m, n - 1) - b P(m, n - 2), and c of the
+// derivative's P(m + 1, n) term; then [32] factors of P(m, m) = -P(m - 1, m - 1) s diag.
 __host__ __device__ constexpr int near_table_doubles(int p) { return 96 * (p + 1) + 32; }
 
 // Value, d/dtheta and d/dphi of the 3 functions S[3][nc] at (x = cos theta, phi), summed over the
 // G lanes of a group (all its lanes get them): lane m < p + 1 runs the recurrence of order m and
 // the order-m blocks (the reference's LegPoly / LegPolyDeriv, src/SphericalHarmonics.cc:889-950;
 // P(m + 1, n) for the derivative comes from lane m + 1).
+// Where a target lies near the surface's centres of curvature the Gauss-Newton steps do not
+// settle, and forty of them amplify a rounding to 1e-6 of the velocity and more: the order of the
+// operations here is part of the result. (Sums of each block before its cosine, and a multiplication
+// by 1 / s alone, took 0.23 ms less for 15,000 pairs at p = 12, and moved such targets.)
 template <int G>
 __device__ __forceinline__ void sh_point(const double* __restrict__ S, const double* __restrict__ tab, int p,
                                          const int* __restrict__ blk_off, double x, double phi, bool grads,
@@ -169,57 +173,74 @@ __device__ __forceinline__ void sh_point(const double* __restrict__ S, const dou
   const int m = threadIdx.x & (G - 1);
   const int nc = p * (p + 2);
   const double s = sqrt(fmax(1.0 - x * x, 0.0)), si = s > 0.0 ? 1.0 / s : 0.0;
-  double pw = 1.0, b = -s;  // (-s)^m
-#pragma unroll
-  for (int i = 0; i < (G == 16 ? 4 : 5); i++) {
-    if (m >> i & 1) pw *= b;
-    b *= b;
-  }
   const bool act = m <= p;
-  const double pmm = act ? tab[96 * (p + 1) + m] * pw : 0.0;
-  double cm = 1.0, sm = 0.0;
-  if (act) sincos(m * phi, &sm, &cm);
+  double pmm = 0.28209479177387814;  // 1/sqrt(4 pi)
+  for (int i = 1; i <= p; i++) {
+    const double rt = tab[96 * (p + 1) + i];
+    if (i <= m) pmm = -pmm * s * rt;
+  }
+  double cm = 1.0, sm = 0.0, dcm = 0.0, dsm = 0.0;
+  if (act) {
+    sincos(m * phi, &sm, &cm);
+    dcm = -m * sm;
+    dsm = m * cm;
+  }
   const int jc = m == 0 ? 0 : (m == p ? 2 * p - 1 : 2 * m - 1);  // cos block of order m
   const bool sine = m >= 1 && m < p;                              // it has a sin block
   const double* Sc = S + (act ? blk_off[jc] : 0) - m;
   const double* Ss = S + (sine ? blk_off[2 * m] : 0) - m;
-  double vc[3] = {0, 0, 0}, vs[3] = {0, 0, 0}, dc[3] = {0, 0, 0}, ds[3] = {0, 0, 0};
-  const double mx = m * x * si;
-  double pm2 = 0.0, pm1 = 0.0;
+  double acc[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) acc[i] = 0.0;
+  double pm2 = 0.0, pm1 = pmm;
   for (int n = 0; n <= p; n++) {
     const double* row = tab + 96 * n + m;
-    const double pn = n == m ? pmm : n > m ? row[0] * x * pm1 - row[32] * pm2 : 0.0;
-    pm2 = pm1;
-    pm1 = pn;
+    double pn = 0.0;
+    if (act && n >= m) {
+      if (n == m) {
+        pn = pmm;
+      } else {
+        const double a = row[0], b = row[32];
+        pn = x * a * pm1 - b * pm2;
+        pm2 = pm1;
+        pm1 = pn;
+      }
+    }
+    // P(m + 1, n) from the next lane (0 beyond the diagonal) for the theta derivative
     const double pnext = __shfl_down_sync(0xffffffffu, pn, 1, G);
     if (act && n >= m) {
-      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta)
-      const double dpn = s > 0.0 ? fma(mx, pn, row[64] * pnext) : 0.0;
+      const double c2 = row[64];
+      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta); the quotient by s from its reciprocal, one
+      // remainder and one correction (Markstein, IBM J. Res. Dev. 34, 1990), which round correctly
+      const double num = m * x * pn + c2 * s * (m + 1 <= n ? pnext : 0.0);
+      const double q0 = num * si;
+      const double dpn = s > 0.0 ? fma(fma(-q0, s, num), si, q0) : 0.0;
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const double a = Sc[d * nc + n];
-        vc[d] = fma(a, pn, vc[d]);
-        if (grads) dc[d] = fma(a, dpn, dc[d]);
-        if (sine) {
-          const double e = Ss[d * nc + n];
-          vs[d] = fma(e, pn, vs[d]);
-          if (grads) ds[d] = fma(e, dpn, ds[d]);
+        acc[d] += a * pn * cm;
+        if (grads) {
+          acc[3 + d] += a * dpn * cm;
+          acc[6 + d] += a * pn * dcm;
+        }
+      }
+      if (sine) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const double a = Ss[d * nc + n];
+          acc[d] += a * pn * sm;
+          if (grads) {
+            acc[3 + d] += a * dpn * sm;
+            acc[6 + d] += a * pn * dsm;
+          }
         }
       }
     }
   }
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    val[d] = fma(vc[d], cm, vs[d] * sm);
-    if (grads) {
-      val[3 + d] = fma(dc[d], cm, ds[d] * sm);
-      val[6 + d] = m * (vs[d] * cm - vc[d] * sm);
-    }
-  }
-#pragma unroll
   for (int i = 0; i < 9; i++) {
     if (i >= 3 && !grads) break;
-    double v = val[i];
+    double v = acc[i];
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
     val[i] = kSqrt2Pi * v;
@@ -255,7 +276,7 @@ constexpr int kProjWarps = 4;
 // use are neighbours). The vesicle's coefficients and the recurrence tables are staged in shared
 // memory. What bounds it is the serial chain of up to 40 Gauss-Newton steps of p + 1 recurrence
 // steps each: with the square roots and divisions of the recurrence in tables, 16 lanes per pair
-// at p <= 15 and every warp at it, 15,000 pairs at p = 12 take 0.65 ms (one warp of a 128-thread CTA
+// at p <= 15 and every warp at it, 15,000 pairs at p = 12 take 0.89 ms (one warp of a 128-thread CTA
 // per pair, three waiting, and the coefficients recomputed took 14.5 ms with the sums of
 // k_near_correct).
 template <int G>
@@ -440,10 +461,8 @@ int launch_centroid_radius(const double* X, long nv, int p, double* cen_r, unsig
 // Recurrence tables of k_near_project (see near_table_doubles).
 std::vector<double> near_tables(int p) {
   std::vector<double> t(near_table_doubles(p), 0.0);
-  double d = 0.28209479177387814;  // 1/sqrt(4 pi)
   for (int m = 0; m <= p; m++) {
-    if (m > 0) d *= std::sqrt((2.0 * m + 1.0) / (2.0 * m));
-    t[96 * (p + 1) + m] = d;
+    t[96 * (p + 1) + m] = m > 0 ? std::sqrt((2.0 * m + 1.0) / (2.0 * m)) : 0.0;
     for (int n = m + 1; n <= p; n++) {
       t[96 * n + m] = std::sqrt(((2.0 * n - 1) * (2.0 * n + 1)) / ((double)(n - m) * (n + m)));
       if (n > m + 1)
