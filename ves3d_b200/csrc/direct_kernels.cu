@@ -146,7 +146,17 @@ static long sum_segments(long M) {
   return std::max(1L, std::min(32L, 16L * 148 / chunks));
 }
 
+// (not monotonic in M: more targets take fewer segments)
 size_t targets_part_doubles(long M) { return sum_segments(M) > 1 ? 3 * (size_t)M * sum_segments(M) : 0; }
+
+// Segments of N sources at M targets with room for part_doubles partial sums.
+long targets_segments(long N, long M, size_t part_doubles, long* tiles_each) {
+  const long room = std::max(1L, (long)(part_doubles / (3 * (size_t)M)));
+  const long tiles = (N + kSumTile - 1) / kSumTile, nseg = std::min(sum_segments(M), room);
+  const long per = std::max(1L, (tiles + nseg - 1) / nseg);
+  if (tiles_each) *tiles_each = per;
+  return std::max(1L, (tiles + per - 1) / per);
+}
 
 int launch_alltoall_f64(const double* pos, const double* den, long np, double* pot, double* part, long slots,
                         cudaStream_t st) {
@@ -378,11 +388,10 @@ int launch_direct_stokes_dl_f64(int src_m, int trg_m, int n, int t_head, int t_t
 // the single layer of den and, with nrm, the double layer of unit normals nrm and densities
 // dden (both densities times area and weights). Few targets split the sources over segments.
 int launch_targets_f64(const double* pos, const double* den, const double* nrm, const double* dden, long N,
-                       const double* trg, long M, double* out, double* part, cudaStream_t st) {
+                       const double* trg, long M, double* out, double* part, size_t part_doubles, cudaStream_t st) {
   if (M <= 0) return VES3D_OK;
-  long nseg = part ? sum_segments(M) : 1;
-  const long tiles = (N + kSumTile - 1) / kSumTile, per = std::max(1L, (tiles + nseg - 1) / nseg);
-  nseg = std::max(1L, (tiles + per - 1) / per);
+  long per = 1;
+  const long nseg = targets_segments(N, M, part_doubles, &per);
   const dim3 grid((unsigned)((M + kSumTrg - 1) / kSumTrg), (unsigned)nseg);
   double* dst = nseg > 1 ? part : out;
   if (nrm)

@@ -165,8 +165,11 @@ int launch_far_dl(bool mixed, const double* pos, const double* nrm, const double
 // layer of den, plus with nrm non-null the double layer of nrm and dden (all point-major,
 // densities times area and weights).
 int launch_targets_f64(const double* pos, const double* den, const double* nrm, const double* dden, long N,
-                       const double* trg, long M, double* out, double* part, cudaStream_t st);
-size_t targets_part_doubles(long M);  // of part, the partial sums of few targets' source segments
+                       const double* trg, long M, double* out, double* part, size_t part_doubles, cudaStream_t st);
+// The doubles of part, the partial sums of few targets' source segments, that M targets ask for; with
+// fewer the launch takes fewer segments.
+size_t targets_part_doubles(long M);
+long targets_segments(long N, long M, size_t part_doubles, long* tiles_each);
 // Unit outward normals (X_theta x X_phi) / |X_theta x X_phi| of nv surfaces at order p0,
 // AxisMajor derivatives in, point-major [N][3] out.
 int launch_unit_normals(const double* Xt, const double* Xp, long nv, int p0, double* nrm, cudaStream_t st);

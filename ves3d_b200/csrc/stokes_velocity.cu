@@ -195,6 +195,7 @@ struct ves3d_sv {
   // off-surface targets (SetTrgCoord): point-major [trg_n][3] and their velocities
   double *trg = nullptr, *vtrg = nullptr, *trg_part = nullptr;  // (trg_part: partial sums)
   long trg_n = 0, trg_cap = 0;
+  size_t trg_part_cap = 0;  // doubles of trg_part
   // near-singular correction of the targets (NearSingular): the upsampled sources of every
   // vesicle (surface, tangents, density, double-layer density at p_up, AxisMajor; area;
   // point-major positions, weighted densities, normals), vesicle centroids and radii,
@@ -849,7 +850,7 @@ int eval_trg_near(ves3d_sv* sv) {
   }
   // the smooth quadrature of every vesicle at every target
   if ((s = launch_targets_f64(sv->nu_pos, sv->nu_den, dl ? sv->nu_nrm : nullptr, dl ? sv->nu_dden : nullptr,
-                              nv * ng1, sv->trg, M, sv->vtrg, sv->trg_part, st)))
+                              nv * ng1, sv->trg, M, sv->vtrg, sv->trg_part, sv->trg_part_cap, st)))
     return s;
   // r_near = r_ves 2 / sqrt(p_up) (src/NearSingular.cc:160, :119-158), formed where it is used
   if ((s = launch_centroid_radius(sv->X, nv, p, sv->nu_cen, sv->nu_rmax, st))) return s;
@@ -1063,13 +1064,19 @@ int ves3d_sv_set_trg_coord(ves3d_sv* sv, const double* T, long n_trg, int is_dev
   if (n_trg > sv->trg_cap) {
     dfree(sv->trg);
     dfree(sv->vtrg);
-    dfree(sv->trg_part);
-    sv->trg = sv->vtrg = sv->trg_part = nullptr;
-    sv->trg_cap = 0;
-    if ((s = dalloc(&sv->trg, 3 * (size_t)n_trg)) || (s = dalloc(&sv->vtrg, 3 * (size_t)n_trg)) ||
-        (s = dalloc(&sv->trg_part, targets_part_doubles(n_trg))))
-      return s;
+    sv->trg = sv->vtrg = nullptr;
+    sv->trg_cap = sv->trg_n = 0;
+    if ((s = dalloc(&sv->trg, 3 * (size_t)n_trg)) || (s = dalloc(&sv->vtrg, 3 * (size_t)n_trg))) return s;
     sv->trg_cap = n_trg;
+  }
+  // the partial sums have a capacity of their own: fewer targets may ask for more of them
+  const size_t part = targets_part_doubles(n_trg);
+  if (part > sv->trg_part_cap) {
+    dfree(sv->trg_part);
+    sv->trg_part = nullptr;
+    sv->trg_part_cap = 0;
+    if ((s = dalloc(&sv->trg_part, part))) return s;
+    sv->trg_part_cap = part;
   }
   if ((s = copy_in(sv->trg, T, 3 * (size_t)n_trg, is_device, sv->stream))) return s;
   sv->trg_n = n_trg;
@@ -1098,7 +1105,7 @@ int ves3d_sv_eval_trg(ves3d_sv* sv, double* vel, int is_device) {
   if (sv->near_on) {
     if ((s = eval_trg_near(sv))) return s;
   } else if ((s = launch_targets_f64(sv->pos, sv->den, nrm, dden, sv->npts(), sv->trg, sv->trg_n, sv->vtrg,
-                                     sv->trg_part, st))) {
+                                     sv->trg_part, sv->trg_part_cap, st))) {
     return s;
   }
   return copy_out(vel, sv->vtrg, 3 * (size_t)sv->trg_n, is_device, st);
