@@ -209,19 +209,27 @@ struct ves3d_sv {
   int *nu_count = nullptr, *nu_v = nullptr, *nu_k = nullptr;
   long nu_ves_cap = 0, nu_trg_cap = 0;
   double near_r = 0.0;  // r_near of the last corrected evaluation
-  void free_near() {
+  // what the vesicles at p_up take, and the tables of that order
+  void free_near_sources() {
     double* ps[] = {nu_X, nu_Xt, nu_Xp, nu_F, nu_G, nu_area, nu_pos, nu_den, nu_nrm, nu_dden, nu_cen, nu_theta, nu_w,
-                    nu_corr, nu_proj, nu_tab};
+                    nu_tab};
     for (double* q : ps) dfree(q);
     nu_X = nu_Xt = nu_Xp = nu_F = nu_G = nu_area = nu_pos = nu_den = nu_nrm = nu_dden = nu_cen = nullptr;
-    nu_theta = nu_w = nu_corr = nu_proj = nu_tab = nullptr;
+    nu_theta = nu_w = nu_tab = nullptr;
+    nu_ves_cap = 0;
+  }
+  void free_near() {
+    free_near_sources();
+    dfree(nu_corr);
+    dfree(nu_proj);
+    nu_corr = nu_proj = nullptr;
     dfree(nu_rmax);
     dfree(nu_count);
     dfree(nu_v);
     dfree(nu_k);
     nu_rmax = nullptr;
     nu_count = nu_v = nu_k = nullptr;
-    nu_ves_cap = nu_trg_cap = 0;
+    nu_trg_cap = 0;
   }
   double *velc = nullptr, *dlc = nullptr;
   long contrast_nves = -1;  // vesicle count the device coefficients were made for
@@ -778,9 +786,7 @@ int eval_trg_near(ves3d_sv* sv) {
   if (dl && !sv->dl_valid && (s = run_setup(sv, true))) return s;
   if ((s = run_self_apply(sv, dl))) return s;  // Fc (Gc) and the self coefficients Vc
   if (sv->nu_ves_cap < nv || (dl && !sv->nu_G)) {
-    double* ps[] = {sv->nu_X, sv->nu_Xt, sv->nu_Xp, sv->nu_F, sv->nu_G, sv->nu_area, sv->nu_pos, sv->nu_den,
-                    sv->nu_nrm, sv->nu_dden, sv->nu_cen, sv->nu_theta, sv->nu_w, sv->nu_tab};
-    for (double* x : ps) dfree(x);
+    sv->free_near_sources();
     const size_t f = (size_t)nv * 3 * ng1;
     s = 0;
     s |= dalloc(&sv->nu_X, f);
@@ -1150,7 +1156,8 @@ int ves3d_sv_set_order_up(ves3d_sv* sv, int sh_order_up) {
   sv->sl_valid = sv->dl_valid = false;  // self matrices of the new order on next use
   sv->parts_valid = false;
   sv->pc_valid = false;
-  sv->free_scratch();  // its size depends on the order
+  sv->free_scratch();  // its size depends on the order, as the near-singular sources' does
+  sv->free_near_sources();
   sv->drop_graph();
   return VES3D_OK;
 }
