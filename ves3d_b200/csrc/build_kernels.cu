@@ -55,11 +55,9 @@ __host__ __device__ constexpr int pad16_4(int n) { return ((n + 11) / 16) * 16 +
 // quarter) takes its kernel and transposed DFT in FP64 on the CUDA cores.
 //
 // Every wait is bounded (about a second of %globaltimer); a wait that runs out sets
-// g_tc_build_error, the CTA stops, waits (bounded) for its copies and MMAs, frees its
+// the caller's error word, the CTA stops, waits (bounded) for its copies and MMAs, frees its
 // TMEM and returns, and the host reports the error.
 // ======================================================================================
-__device__ int g_tc_build_error = 0;
-
 namespace tc {
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -377,7 +375,7 @@ __device__ __forceinline__ void ring_kernel_sl_f32(float px, float py, float pz,
 
 template <int P0>
 __global__ void __launch_bounds__(512, 1) k_build_ring_tc(const double* __restrict__ R, DevTables T,
-                                                          float* __restrict__ C, long nrot) {
+                                                          float* __restrict__ C, long nrot, int* err) {
   using H = RingTcCfg<P0>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* sB12 = smem + H::OFF_B12;
@@ -476,7 +474,7 @@ __global__ void __launch_bounds__(512, 1) k_build_ring_tc(const double* __restri
   bool ok = true;
   auto wait = [&](uint64_t* bar, uint32_t& cnt) {
     if (!tc::mbar_wait(bar, cnt & 1)) {
-      atomicExch(&g_tc_build_error, 1);
+      atomicExch(err, 1);
       *s_abort = 1;
     }
     cnt++;
@@ -859,7 +857,7 @@ __global__ void __launch_bounds__(512, 1) k_build_ring_tc(const double* __restri
     auto drain = [&](uint64_t* bar, uint32_t& waited, uint32_t issued) {
       while (drained && waited < issued) {
         if (!tc::mbar_wait(bar, waited & 1)) {
-          atomicExch(&g_tc_build_error, 1);
+          atomicExch(err, 1);
           drained = false;
         }
         waited++;
@@ -879,7 +877,7 @@ __global__ void __launch_bounds__(512, 1) k_build_ring_tc(const double* __restri
 
 bool tc_build_supported(int p0, int p1) { return p0 == 16 && p1 == 32; }
 
-int launch_build_ring_tc(const double* R, long nrot, const DevTables& T, float* C, cudaStream_t st) {
+int launch_build_ring_tc(const double* R, long nrot, const DevTables& T, float* C, int* err, cudaStream_t st) {
   if (nrot <= 0) return VES3D_OK;
   if (!tc_build_supported(T.p0, T.p1)) {
     set_error("tensor-core build not laid out for p = %d, p_up = %d", T.p0, T.p1);
@@ -895,19 +893,9 @@ int launch_build_ring_tc(const double* R, long nrot, const DevTables& T, float* 
   VES3D_CK(cudaGetDevice(&dev));
   VES3D_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const long grid = std::min(nrot, (long)nsm);
-  k_build_ring_tc<16><<<(unsigned)grid, H::NTHR, H::SMEM, st>>>(R, T, C, nrot);
+  k_build_ring_tc<16><<<(unsigned)grid, H::NTHR, H::SMEM, st>>>(R, T, C, nrot, err);
   VES3D_LAUNCHED();
   return VES3D_OK;
-}
-
-int tc_build_error(bool reset) {
-  int v = 0;
-  VES3D_CK(cudaMemcpyFromSymbol(&v, g_tc_build_error, sizeof(int)));
-  if (v && reset) {
-    const int zero = 0;
-    VES3D_CK(cudaMemcpyToSymbol(g_tc_build_error, &zero, sizeof(int)));
-  }
-  return v;
 }
 
 }  // namespace ves3d

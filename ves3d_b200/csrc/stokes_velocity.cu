@@ -281,7 +281,11 @@ struct ves3d_sv {
   // where the call waits for its result anyway (collect_times): the host queues a whole evaluation
   // without stopping between its stages.
   cudaEvent_t ev[12] = {}, ev_copied = nullptr, ev_src = nullptr;  // (ev_src: the surfaces' fields are formed)
-  bool t_setup = false, t_setup_dl = false, t_eval = false, t_eval_dl = false, check_tc = false;
+  bool t_setup = false, t_setup_dl = false, t_eval = false, t_eval_dl = false;
+  // a tensor-core build was queued whose error word (this context's own, so that several contexts may
+  // have builds in flight) has not been read yet
+  bool check_tc = false;
+  int* tc_err = nullptr;
   float ms[4] = {0, 0, 0, 0};
   float far_dl_ms = 0;  // the far double layer's segment kernels in the last evaluation
 
@@ -293,6 +297,7 @@ struct ves3d_sv {
     dfree(trg);
     dfree(vtrg);
     dfree(trg_part);
+    dfree(tc_err);
     drop_graph();
     free_precond();
     for (auto& e : pc_ev)
@@ -551,11 +556,17 @@ int collect_times(ves3d_sv* sv) {
   }
   if (sv->check_tc) {
     sv->check_tc = false;
-    if (tc_build_error(true)) {
-      sv->sl_valid = false;
+    const bool valid = sv->sl_valid;
+    sv->sl_valid = false;  // until the word is read
+    int err = 0;
+    VES3D_CK(cudaMemcpyAsync(&err, sv->tc_err, sizeof(int), cudaMemcpyDeviceToHost, sv->stream));
+    VES3D_CK(cudaStreamSynchronize(sv->stream));
+    if (err) {
+      VES3D_CK(cudaMemsetAsync(sv->tc_err, 0, sizeof(int), sv->stream));
       set_error("self-matrix build on the tensor cores: a bounded wait of the kernel ran out");
       return VES3D_ERR_CUDA;
     }
+    sv->sl_valid = valid;
   }
   return VES3D_OK;
 }
@@ -578,6 +589,10 @@ int run_setup(ves3d_sv* sv, bool dl, bool wait) {
     set_error("internal: self-matrix build without its buffers");
     return VES3D_ERR_STATE;
   }
+  if (tc && !sv->tc_err) {
+    if ((s = dalloc(&sv->tc_err, 1))) return s;
+    VES3D_CK(cudaMemsetAsync(sv->tc_err, 0, sizeof(int), st));
+  }
   VES3D_CK(cudaEventRecord(sv->ev[dl ? 10 : 0], st));
   for (long v0 = 0; v0 < sv->nves; v0 += sv->chunk) {
     const long nb = std::min(sv->chunk, sv->nves - v0);
@@ -587,7 +602,7 @@ int run_setup(ves3d_sv* sv, bool dl, bool wait) {
     // rotated back in FP32; the FP64 builds leave FP64 ones
     float* Cf = reinterpret_cast<float*>(sv->C);
     if (fused && tc) {
-      if ((s = launch_build_ring_tc(sv->R, nrot, T, Cf, st))) return s;
+      if ((s = launch_build_ring_tc(sv->R, nrot, T, Cf, sv->tc_err, st))) return s;
     } else if (fused) {
       if ((s = launch_ring_build(dl, sv->R, nrot, T, sv->C, st))) return s;
     } else {
@@ -734,10 +749,7 @@ int run_eval_body(ves3d_sv* sv, bool dl) {
   return join_far(sv, nseg, dl);
 }
 
-// One evaluation; dl adds the double layer of the density G (the operator's own
-// evaluation when a double-layer density is set; the implicit step applies the single
-// layer alone). wait: until it is done (else it is queued, its times left to collect_times).
-int run_eval(ves3d_sv* sv, bool dl, bool wait = true) {
+int queue_eval(ves3d_sv* sv, bool dl) {
   cudaStream_t st = sv->stream;
   int s, nseg = 0;
   if (!sv->have_src || !sv->have_den) {
@@ -761,8 +773,20 @@ int run_eval(ves3d_sv* sv, bool dl, bool wait = true) {
   VES3D_CK(cudaEventRecord(sv->ev[6], st));
   sv->t_eval = true;
   sv->t_eval_dl = dl;
-  // (the tensor-core build's result is checked before it is used further)
-  if ((wait || sv->check_tc) && (s = collect_times(sv))) return s;
+  return VES3D_OK;
+}
+
+// One evaluation; dl adds the double layer of the density G (the operator's own
+// evaluation when a double-layer density is set; the implicit step applies the single
+// layer alone). wait: until it is done (else it is queued, its times left to collect_times).
+int run_eval(ves3d_sv* sv, bool dl, bool wait = true) {
+  int s = queue_eval(sv, dl);
+  // (the tensor-core build's result is checked before it is used further, whatever followed it)
+  if ((wait && !s) || sv->check_tc) {
+    const int e = collect_times(sv);
+    if (!s) s = e;
+  }
+  if (s) return s;
   sv->parts_valid = true;
   return VES3D_OK;
 }
@@ -3466,13 +3490,7 @@ int ves3d_svp_launch_eval_graph(ves3d_svp* g, double* vel, int is_device) {
   return vel ? copy_out(vel, g->V, 3 * (size_t)g->N, is_device, g->stream) : VES3D_OK;
 }
 
-int ves3d_svp_eval(ves3d_svp* g, double* vel, int is_device) {
-  VES3D_ARG(g && vel, "null argument");
-  if (g->grp.empty() || !g->have_den) {
-    set_error("eval before set_src_coord / set_density_sl");
-    return VES3D_ERR_STATE;
-  }
-  VES3D_CK(cudaSetDevice(g->device));
+static int svp_queue_eval(ves3d_svp* g) {
   int s;
   VES3D_CK(cudaEventRecord(g->ev[0], g->stream));
   if ((s = svp_setup(g, /*wait=*/false))) return s;
@@ -3482,13 +3500,41 @@ int ves3d_svp_eval(ves3d_svp* g, double* vel, int is_device) {
   if ((s = svp_far(g, g->have_dl))) return s;
   VES3D_CK(cudaEventRecord(g->ev[3], g->stream));
   VES3D_CK(cudaEventSynchronize(g->ev[3]));
-  for (ves3d_sv* sv : g->grp)
-    if ((s = collect_times(sv))) return s;
+  return VES3D_OK;
+}
+
+int ves3d_svp_eval(ves3d_svp* g, double* vel, int is_device) {
+  VES3D_ARG(g && vel, "null argument");
+  if (g->grp.empty() || !g->have_den) {
+    set_error("eval before set_src_coord / set_density_sl");
+    return VES3D_ERR_STATE;
+  }
+  VES3D_CK(cudaSetDevice(g->device));
+  int s = svp_queue_eval(g);
+  for (ves3d_sv* sv : g->grp) {  // every group's build is checked, whatever became of the others
+    const int e = collect_times(sv);
+    if (!s) s = e;
+  }
+  if (s) return s;
   VES3D_CK(cudaEventElapsedTime(&g->ms[0], g->ev[0], g->ev[1]));
   VES3D_CK(cudaEventElapsedTime(&g->ms[1], g->ev[1], g->ev[2]));
   VES3D_CK(cudaEventElapsedTime(&g->ms[2], g->ev[2], g->ev[3]));
   VES3D_CK(cudaEventElapsedTime(&g->ms[3], g->ev[0], g->ev[3]));
   return copy_out(vel, g->V, 3 * (size_t)g->N, is_device, g->stream);
+}
+
+// For tests, not part of the interface: whether an order group's self matrices count as built (1 or 0),
+// and with fail the error word of its tensor-core build set as a bounded wait that runs out sets it.
+int ves3d_svp_test_build_error(ves3d_svp* g, int group, int fail) {
+  VES3D_ARG(g && group >= 0 && group < (int)g->grp.size(), "no such group");
+  ves3d_sv* sv = g->grp[group];
+  const int one = 1;
+  if (fail) {
+    if (!sv->tc_err) return -1;
+    VES3D_CK(cudaMemcpyAsync(sv->tc_err, &one, sizeof(int), cudaMemcpyHostToDevice, g->stream));
+    VES3D_CK(cudaStreamSynchronize(g->stream));
+  }
+  return sv->sl_valid;
 }
 
 int ves3d_svp_stage_times(ves3d_svp* g, float* ms) {
