@@ -18,6 +18,8 @@
 
 namespace ves3d {
 
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory a CTA may have
+
 __global__ void __launch_bounds__(256) k_analysis(const double* __restrict__ in, long nfun, int nlat, int nlon,
                                                   int nfo, const double* __restrict__ four,
                                                   const double* __restrict__ leg, const int* __restrict__ jf,
@@ -56,7 +58,10 @@ __global__ void __launch_bounds__(256) k_analysis(const double* __restrict__ in,
 // values, one coefficient broadcast) and one table value for the CTA's functions; the DFT takes lanes
 // along the longitudes, four latitudes per thread on one table value. Bound by the table reads from
 // L1: a load per multiply-add before (1,536 functions of p = 16: 260 us), one per FB or four now (71 us).
-template <int FB>
+// PAD: the latitudes of a row padded to whole groups of four, read in 16-byte loads. Without (orders whose
+// padded rows outgrow shared memory) the last group of a row reads on into what follows it, for sums that
+// are not stored.
+template <int FB, bool PAD>
 __global__ void __launch_bounds__(256) k_synthesis(const double* __restrict__ S, long nfun, int nci, int nfi,
                                                    int nlat, int nlon, const double* __restrict__ leg,
                                                    const double* __restrict__ dleg,
@@ -66,7 +71,7 @@ __global__ void __launch_bounds__(256) k_synthesis(const double* __restrict__ S,
                                                    double* __restrict__ X, double* __restrict__ Xt,
                                                    double* __restrict__ Xp) {
   extern __shared__ __align__(16) double sm[];
-  const int nls = (nlat + 3) & ~3;                  // latitudes padded to whole groups of four
+  const int nls = PAD ? (nlat + 3) & ~3 : nlat;     // row stride
   double* sb = sm;                                  // [FB][nfi][nls]
   double* sd = sb + (size_t)FB * nfi * nls;         // the same of dleg (if Xp)
   double* ss = sd + (Xp ? (size_t)FB * nfi * nls : 0);  // [FB][nci]
@@ -98,7 +103,19 @@ __global__ void __launch_bounds__(256) k_synthesis(const double* __restrict__ S,
     }
   }
   __syncthreads();
-  const int ngr = nls / 4;
+  const int ngr = (nlat + 3) / 4;
+  auto four_of = [](const double* a, double (&v)[4]) {
+    if (PAD) {
+      const double2 b0 = reinterpret_cast<const double2*>(a)[0], b1 = reinterpret_cast<const double2*>(a)[1];
+      v[0] = b0.x;
+      v[1] = b0.y;
+      v[2] = b1.x;
+      v[3] = b1.y;
+    } else {
+#pragma unroll
+      for (int l = 0; l < 4; l++) v[l] = a[l];
+    }
+  };
   for (int i = threadIdx.x; i < nf * ngr * nlon; i += blockDim.x) {
     const int j = i % nlon, r = i / nlon, f = r / ngr, lat0 = 4 * (r - f * ngr);
     const double* br = sb + (size_t)f * nfi * nls + lat0;
@@ -107,21 +124,18 @@ __global__ void __launch_bounds__(256) k_synthesis(const double* __restrict__ S,
 #pragma unroll 4
     for (int k = 0; k < nfi; k++) {
       const double w = __ldg(four + k * nlon + j), dw = Xt ? __ldg(dfour + k * nlon + j) : 0.0;
-      const double2 b0 = *reinterpret_cast<const double2*>(br + k * nls);
-      const double2 b1 = *reinterpret_cast<const double2*>(br + k * nls + 2);
-      const double b[4] = {b0.x, b0.y, b1.x, b1.y};
+      double b[4];
+      four_of(br + k * nls, b);
 #pragma unroll
       for (int l = 0; l < 4; l++) x[l] = fma(b[l], w, x[l]);
       if (Xt)
 #pragma unroll
         for (int l = 0; l < 4; l++) xt[l] = fma(b[l], dw, xt[l]);
       if (Xp) {
-        const double2 d0 = *reinterpret_cast<const double2*>(dr + k * nls);
-        const double2 d1 = *reinterpret_cast<const double2*>(dr + k * nls + 2);
-        xp[0] = fma(d0.x, w, xp[0]);
-        xp[1] = fma(d0.y, w, xp[1]);
-        xp[2] = fma(d1.x, w, xp[2]);
-        xp[3] = fma(d1.y, w, xp[3]);
+        double d[4];
+        four_of(dr + k * nls, d);
+#pragma unroll
+        for (int l = 0; l < 4; l++) xp[l] = fma(d[l], w, xp[l]);
       }
     }
 #pragma unroll
@@ -166,13 +180,18 @@ int launch_synthesis(const double* S, long nfun, int p0, int q, const double* le
                      const double* four, const double* dfour, const int* blk_off, double* X, double* Xt,
                      double* Xp, cudaStream_t st) {
   if (nfun <= 0) return VES3D_OK;
-  const int nci = ncoef_(p0), nfi = 2 * p0, nlat = q + 1, nlon = 2 * q, nls = (nlat + 3) & ~3;
-  const size_t per = ((size_t)nci + (size_t)nls * nfi * (Xp ? 2 : 1)) * sizeof(double);
+  const int nci = ncoef_(p0), nfi = 2 * p0, nlat = q + 1, nlon = 2 * q;
+  auto bytes = [&](int nls) { return ((size_t)nci + (size_t)nls * nfi * (Xp ? 2 : 1)) * sizeof(double); };
+  const bool pad = bytes((nlat + 3) & ~3) <= kMaxSmem;
+  const size_t per = bytes(pad ? (nlat + 3) & ~3 : nlat);
   // functions per CTA: as many as leave two CTAs per SM to run and 96 KB to a CTA
   int fb = 4;
   while (fb > 1 && (nfun < 2L * 148 * fb || per * fb > 96 * 1024)) fb /= 2;
   const size_t smem = per * fb;
-  auto kernel = fb == 4 ? k_synthesis<4> : fb == 2 ? k_synthesis<2> : k_synthesis<1>;
+  auto kernel = fb == 4   ? k_synthesis<4, true>
+                : fb == 2 ? k_synthesis<2, true>
+                : pad     ? k_synthesis<1, true>
+                          : k_synthesis<1, false>;
   if (smem > 48 * 1024) VES3D_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kernel<<<(unsigned)((nfun + fb - 1) / fb), 256, smem, st>>>(S, nfun, nci, nfi, nlat, nlon, leg, dleg, four, dfour,
                                                               blk_off, X, Xt, Xp);
