@@ -35,6 +35,18 @@ inline int cuda_status(cudaError_t e, const char* what, const char* file, int li
     if (_st != VES3D_OK) return _st;                                            \
   } while (0)
 
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory a CTA may have
+
+// Opt a kernel without static shared memory in to all of it, whatever this launch takes: the attribute is
+// the kernel's, not the launch's, and a smaller value that another thread sets for its own size between
+// here and the launch would refuse this one.
+template <class K>
+inline int allow_smem(K kernel, size_t smem) {
+  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(smem > kMaxSmem ? smem : kMaxSmem)),
+                     "shared memory of a kernel", __FILE__, __LINE__);
+}
+
 #define VES3D_ARG(cond, msg)                                                    \
   do {                                                                          \
     if (!(cond)) {                                                              \

@@ -488,7 +488,7 @@ template <int G>
 static int launch_project(const NearArgs& a, cudaStream_t st) {
   const int per = 32 * kProjWarps / G, p = a.p;
   const size_t smem = ((size_t)near_table_doubles(p) + p + 1 + (size_t)per * 3 * p * (p + 2)) * sizeof(double);
-  VES3D_CK(cudaFuncSetAttribute(k_near_project<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int s = allow_smem(k_near_project<G>, smem)) return s;
   k_near_project<G><<<(unsigned)((a.M * kNearMax + per - 1) / per), 32 * kProjWarps, smem, st>>>(a);
   VES3D_LAUNCHED();
   return VES3D_OK;

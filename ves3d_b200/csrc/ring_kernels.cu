@@ -543,7 +543,7 @@ int launch_ring(const double* R, long nrot, const DevTables& T, double* C, cudaS
     set_error("internal: fused self-matrix build at p = %d, p_up = %d needs %zu bytes of shared memory", T.p0, T.p1, smem);
     return VES3D_ERR_ARG;
   }
-  VES3D_CK(cudaFuncSetAttribute(k_ring<P, GEN, DL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int s = allow_smem(k_ring<P, GEN, DL>, smem)) return s;
   int dev = 0, nsm = 148, per = 1;
   VES3D_CK(cudaGetDevice(&dev));
   VES3D_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

@@ -285,7 +285,7 @@ int launch_sht_mode(ShtArgs a, cudaStream_t st) {
   while (fb > 1 && bytes(fb) > 200 * 1024) fb--;
   a.fb = fb;
   const size_t smem = bytes(fb);
-  VES3D_CK(cudaFuncSetAttribute(k_sht<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int s = allow_smem(k_sht<MODE>, smem)) return s;
   int per = 1;
   VES3D_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sht<MODE>, kShtThreads, smem));
   const long grid = std::min((a.nfun + fb - 1) / fb, (long)nsm * std::max(per, 1));

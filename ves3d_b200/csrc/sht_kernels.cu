@@ -18,8 +18,6 @@
 
 namespace ves3d {
 
-constexpr size_t kMaxSmem = 227 * 1024;  // shared memory a CTA may have
-
 __global__ void __launch_bounds__(256) k_analysis(const double* __restrict__ in, long nfun, int nlat, int nlon,
                                                   int nfo, const double* __restrict__ four,
                                                   const double* __restrict__ leg, const int* __restrict__ jf,
@@ -169,7 +167,8 @@ int launch_analysis(const double* in, long nfun, int pin, int pout, const double
   const int nlat = pin + 1, nlon = 2 * pin, nfo = 2 * pout, nco = ncoef_(pout);
   const int fpb = pick_fpb((size_t)nlat * (nlon + nfo), nfun);
   size_t smem = (size_t)fpb * nlat * (nlon + nfo) * sizeof(double);
-  if (smem > 48 * 1024) VES3D_CK(cudaFuncSetAttribute(k_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024)
+    if (const int s = allow_smem(k_analysis, smem)) return s;
   long nblk = (nfun + fpb - 1) / fpb;
   k_analysis<<<(unsigned)nblk, 256, smem, st>>>(in, nfun, nlat, nlon, nfo, four, leg, jf, nco, fpb, out);
   VES3D_LAUNCHED();
@@ -192,7 +191,8 @@ int launch_synthesis(const double* S, long nfun, int p0, int q, const double* le
                 : fb == 2 ? k_synthesis<2, true>
                 : pad     ? k_synthesis<1, true>
                           : k_synthesis<1, false>;
-  if (smem > 48 * 1024) VES3D_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024)
+    if (const int s = allow_smem(kernel, smem)) return s;
   kernel<<<(unsigned)((nfun + fb - 1) / fb), 256, smem, st>>>(S, nfun, nci, nfi, nlat, nlon, leg, dleg, four, dfour,
                                                               blk_off, X, Xt, Xp);
   VES3D_LAUNCHED();

@@ -179,7 +179,7 @@ int launch_rotate_all(const double* S, long nv, const DevTables& T, double* R, c
   const dim3 grid(p0 + 1, (unsigned)nv, (unsigned)parts);
   const int nt = ((int)nc + 31) / 32 * 32;
   auto launch = [&](auto kernel) {
-    VES3D_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (const int s = allow_smem(kernel, smem)) return s;
     kernel<<<grid, nt, smem, st>>>(S, p0, mpt, T, R);
     return (int)VES3D_OK;
   };
@@ -766,7 +766,7 @@ int launch_rotate_transpose_scatter(const double* C, long nv, const DevTables& T
       const int rows8 = ((cb * p0) + 7) & ~7;
       const size_t smem = ((size_t)rows8 * ldi + 4 * p0) * sizeof(double) + ((size_t)nc * 5 + 15) / 16 * 16;
       if (p0 <= 16 && smem <= 113 * 1024 && !tc_rotate_disabled()) {
-        VES3D_CK(cudaFuncSetAttribute(k_rotate_transpose_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (const int s = allow_smem(k_rotate_transpose_tc, smem)) return s;
         dim3 grid(p0 + 1, (unsigned)nv);
         k_rotate_transpose_tc<<<grid, 256, smem, st>>>(C, p0, cb, ldi, T, SL3);
         VES3D_LAUNCHED();
@@ -783,7 +783,7 @@ int launch_rotate_transpose_scatter(const double* C, long nv, const DevTables& T
   if (jb < kRtJ) jb = kRtJ;
   size_t smem = ((size_t)2 * jb * (nc + 2) + mpt) * sizeof(double);
   if (smem > 48 * 1024)
-    VES3D_CK(cudaFuncSetAttribute(k_rotate_transpose_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (const int s = allow_smem(k_rotate_transpose_scatter, smem)) return s;
   dim3 grid(p0 + 1, (unsigned)nv);
   k_rotate_transpose_scatter<<<grid, 256, smem, st>>>(C, p0, jb, mpt, T, SL3);
   VES3D_LAUNCHED();
@@ -893,11 +893,11 @@ int launch_self_gemv_multi(const double* F, const double* SL, long nv, int nvec,
   const size_t smem = (size_t)nvec * n * sizeof(double);
   if (accumulate) {
     if (smem > 48 * 1024)
-      VES3D_CK(cudaFuncSetAttribute(k_self_gemv_multi<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (const int s = allow_smem(k_self_gemv_multi<true>, smem)) return s;
     k_self_gemv_multi<true><<<grid, 128, smem, st>>>(F, SL, nv, nvec, n, V);
   } else {
     if (smem > 48 * 1024)
-      VES3D_CK(cudaFuncSetAttribute(k_self_gemv_multi<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (const int s = allow_smem(k_self_gemv_multi<false>, smem)) return s;
     k_self_gemv_multi<false><<<grid, 128, smem, st>>>(F, SL, nv, nvec, n, V);
   }
   VES3D_LAUNCHED();
