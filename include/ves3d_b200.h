@@ -156,14 +156,16 @@ int ves3d_sv_launch_eval_graph(ves3d_sv* sv);
  * default (or VES3D_AUTOTUNE=1): on the first far-field launch of a configuration
  * (precision, points, vesicles and their sizes) every candidate shape -- waves of CTAs
  * per SM in {4, 8, 16} x threads per CTA in {256, 384} (two targets each; the mixed form
- * 256 only, for its accuracy) -- is timed once with CUDA events and the fastest is kept.
+ * 256 only, for its accuracy) -- is timed once with CUDA events beside the default shape
+ * and the fastest of them all is kept.
  * FP64 sums over 8000 and more points have one form that needs no tuning (every unordered
  * pair evaluated once) unless a shape is fixed. Never tunes during stream capture. */
 int ves3d_set_autotune(int on);
 /* Fix the far-field launch shape instead (waves in {4, 8, 16}, threads per CTA in
  * {256, 384}, targets per thread 2); waves = 0 returns to the default / autotuned shape. */
 int ves3d_set_far_shape(int waves, int threads, int targets_per_thread);
-/* Text report of the tuned configurations, one line each ("key waves=W threads=T ms=M");
+/* Text report of the tuned configurations, one line each: the fastest candidate as
+ * "key waves=W threads=T ms=M", followed by " default=1" where the default shape was faster;
  * *len receives its length (buf may be NULL). */
 int ves3d_autotune_report(char* buf, size_t cap, size_t* len);
 

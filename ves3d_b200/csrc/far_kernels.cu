@@ -812,15 +812,17 @@ static int launch_far_shape(const FarShape& sh, bool mixed, const double* pos, c
 
 // ---- autotuner of the launch shape ----------------------------------------------------
 // On the first launch of a configuration (precision, N, vesicles and their sizes) with
-// autotuning on, every candidate shape is launched once and timed with CUDA events on the
-// caller's stream; the fastest is cached for the process. Off by default and never during
+// autotuning on, every candidate shape and the default one are launched once and timed with CUDA
+// events on the caller's stream; the fastest is cached for the process (the report tells the fastest
+// candidate, and whether the default shape was faster). Off by default and never during
 // stream capture. Candidates differ in how the source range is split and in the chunks of
 // targets, i.e. in the grouping of the FP64 partial sums (and, in the FP32 form, in the
 // origin of a chunk's coordinates): results agree to rounding. A tuned configuration
 // always uses its one shape afterwards, so repeated evaluations stay bitwise identical.
 struct FarTuneEntry {
-  FarShape shape;
+  FarShape shape;  // the fastest candidate and its time
   float ms = 0;
+  bool keep_default = false;
 };
 
 static std::mutex g_tune_mu;
@@ -875,7 +877,7 @@ static int tuned_shape(bool mixed, const double* pos, const double* den, const l
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) {
-      *shape = it->second.shape;
+      if (!it->second.keep_default) *shape = it->second.shape;
       return VES3D_OK;
     }
   }
@@ -886,28 +888,35 @@ static int tuned_shape(bool mixed, const double* pos, const double* den, const l
   FarTuneEntry best;
   best.ms = 1e30f;
   int s = VES3D_OK;
+  auto timed = [&](const FarShape& c, float* ms) {
+    int nseg = 0;
+    cudaEventRecord(e0, st);
+    if ((s = launch_far_shape(c, mixed, pos, den, off, nves, N, part, part_cap_segments, st, &nseg))) return false;
+    cudaEventRecord(e1, st);
+    cudaEventSynchronize(e1);
+    cudaEventElapsedTime(ms, e0, e1);
+    return true;
+  };
   for (int nthr : {256, 384})
     for (int waves : {4, 8, 16}) {
-      if (mixed && nthr != 256) continue;
+      if (s || (mixed && nthr != 256)) continue;
       const FarShape c{waves, nthr};
-      cudaEventRecord(e0, st);
-      int nseg = 0;
-      if ((s = launch_far_shape(c, mixed, pos, den, off, nves, N, part, part_cap_segments, st, &nseg))) break;
-      cudaEventRecord(e1, st);
-      cudaEventSynchronize(e1);
       float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best.ms) {
+      if (timed(c, &ms) && ms < best.ms) {
         best.ms = ms;
         best.shape = c;
       }
     }
+  if (!s && !mixed) {  // (the mixed form's default is among the candidates)
+    float ms = 0;
+    best.keep_default = timed(*shape, &ms) && ms <= best.ms;
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (s) return s;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tuned[key] = best;
-  *shape = best.shape;
+  if (!best.keep_default) *shape = best.shape;
   return VES3D_OK;
 }
 
@@ -949,7 +958,8 @@ std::string autotune_report() {
   std::string r;
   for (const auto& kv : g_tuned)
     r += kv.first + " waves=" + std::to_string(kv.second.shape.waves) + " threads=" +
-         std::to_string(kv.second.shape.nthr) + " ms=" + std::to_string(kv.second.ms) + "\n";
+         std::to_string(kv.second.shape.nthr) + " ms=" + std::to_string(kv.second.ms) +
+         (kv.second.keep_default ? " default=1" : "") + "\n";
   return r;
 }
 
