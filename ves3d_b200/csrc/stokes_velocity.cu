@@ -474,12 +474,9 @@ size_t scratch_per_vesicle(int p0, int p1, bool fused) {
 
 int alloc_scratch(ves3d_sv* sv) {
   const long want = sv->nves;
-  // the double layer is built stage by stage: those stage buffers are kept while a
-  // double-layer density is set (the fused single-layer build needs a subset of them)
-  const bool stages = !use_fused(sv) || sv->have_dl || sv->contrast;
-  const bool layout_ok = !stages || sv->K != nullptr;
+  const bool fused = use_fused(sv);  // of both layers; else the stage buffers as well
+  const bool layout_ok = fused || sv->K != nullptr;
   if (sv->chunk >= want && layout_ok) return VES3D_OK;  // the whole suspension in one chunk already
-  const bool fused = !stages;
   size_t per = scratch_per_vesicle(sv->p, sv->pup, fused) * sizeof(double);
   size_t free_b = 0, total_b = 0;
   VES3D_CK(cudaMemGetInfo(&free_b, &total_b));
@@ -3370,7 +3367,7 @@ int ves3d_svp_set_density_dl(ves3d_svp* g, const double* gdl, int is_device) {
     return VES3D_OK;
   }
   if ((s = svp_alloc_dl(g))) return s;
-  // each group's own SetDensityDL: its G buffer, and the stage buffers its DL build needs
+  // each group's own SetDensityDL: its G buffer
   for (size_t r = 0; r < g->grp.size(); r++)
     if ((s = ves3d_sv_set_density_dl(g->grp[r], gdl + 3 * g->gpt0[r], is_device))) return s;
   if (!g->have_dl) g->drop_graph();  // a captured evaluation without the double layer
