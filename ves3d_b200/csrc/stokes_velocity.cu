@@ -158,6 +158,33 @@ struct TablesOwner {
 
 using namespace ves3d;
 
+// Sets of far-field partial sums, of each form that a context runs: the FP32 form (mixed) writes at most
+// kFarMaxSegments of them, the FP64 one far_slots. Each is made when its form first runs (outside any
+// stream capture, which an eager evaluation precedes) and keeps its address, which a captured evaluation
+// holds, until the points outgrow it.
+struct FarPart {
+  double* buf[2] = {nullptr, nullptr};  // FP64, FP32
+  size_t doubles[2] = {0, 0};
+  void free() {
+    for (int i = 0; i < 2; i++) {
+      dfree(buf[i]);
+      buf[i] = nullptr;
+      doubles[i] = 0;
+    }
+  }
+  // the form's buffer, made for cap_points points, and the sets of N points that it holds
+  int get(bool f32, long N, long cap_points, double** part, long* sets) {
+    if (!buf[f32]) {
+      const size_t n = (size_t)(f32 ? kFarMaxSegments : far_slots(cap_points)) * 3 * cap_points;
+      if (int s = dalloc(&buf[f32], n)) return s;
+      doubles[f32] = n;
+    }
+    *part = buf[f32];
+    *sets = (long)(doubles[f32] / (3 * (size_t)N));
+    return VES3D_OK;
+  }
+};
+
 constexpr int kPcStreams = 32;  // streams of the preconditioner factorisation
 constexpr int kPcBatch = 8;     // operator columns per application in its assembly
 
@@ -179,11 +206,13 @@ struct ves3d_sv {
   // resident buffers
   double *X = nullptr, *F = nullptr, *V = nullptr, *Vself = nullptr, *Vfar = nullptr;
   double *Sx = nullptr, *Xt = nullptr, *Xp = nullptr, *area = nullptr, *pos = nullptr, *den = nullptr;
-  double *SL = nullptr, *Fc = nullptr, *Vc = nullptr, *part = nullptr;
+  double *SL = nullptr, *Fc = nullptr, *Vc = nullptr;
+  FarPart far_sl, far_dl;                        // partial sums of the far field's two layers
+  double *part = nullptr, *part_dl = nullptr;  // those of the evaluation under way
   // double layer (allocated when a double-layer density is first set): density G and its
   // coefficients Gc, the self matrices DL, unit normals and weighted densities of the far
-  // sum (point-major) and its segment partials
-  double *G = nullptr, *Gc = nullptr, *DL = nullptr, *nrm = nullptr, *dden = nullptr, *part_dl = nullptr;
+  // sum (point-major)
+  double *G = nullptr, *Gc = nullptr, *DL = nullptr, *nrm = nullptr, *dden = nullptr;
   long dl_cap = 0;
   bool have_dl = false, dl_valid = false;
   int nseg_dl = 0;
@@ -318,19 +347,21 @@ struct ves3d_sv {
     if (own_stream) cudaStreamDestroy(own_stream);
   }
   void free_dl() {
-    double* ps[] = {G, Gc, DL, nrm, dden, part_dl};
+    double* ps[] = {G, Gc, DL, nrm, dden};
     for (double* q : ps) dfree(q);
-    G = Gc = DL = nrm = dden = part_dl = nullptr;
+    G = Gc = DL = nrm = dden = nullptr;
+    far_dl.free();
     dl_cap = 0;
     have_dl = dl_valid = false;
   }
   void free_buffers() {
     free_dl();
-    double* ps[] = {X, F, V, Vself, Vfar, Sx, Xt, Xp, area, pos, den, SL, Fc, Vc, part};
+    double* ps[] = {X, F, V, Vself, Vfar, Sx, Xt, Xp, area, pos, den, SL, Fc, Vc};
     for (double* q : ps) dfree(q);
+    far_sl.free();
     dfree(off);
     off = nullptr;
-    X = F = V = Vself = Vfar = Sx = Xt = Xp = area = pos = den = SL = Fc = Vc = part = nullptr;
+    X = F = V = Vself = Vfar = Sx = Xt = Xp = area = pos = den = SL = Fc = Vc = nullptr;
     cap_ves = 0;
     off_nves = -1;
   }
@@ -361,11 +392,6 @@ struct ves3d_sv {
     chunk = 0;
   }
   long npts() const { return nves * ngrid_(p); }
-  // sets of far-field partial sums of the current points that the buffers (sized for cap_ves) hold
-  long part_slots() const {
-    const long cap = cap_ves * ngrid_(p);
-    return far_slots(cap) * cap / npts();
-  }
 };
 
 namespace {
@@ -419,7 +445,6 @@ int alloc_dl(ves3d_sv* sv) {
   s |= dalloc(&sv->DL, (size_t)nves * n * n);
   s |= dalloc(&sv->nrm, fld);
   s |= dalloc(&sv->dden, fld);
-  s |= dalloc(&sv->part_dl, (size_t)far_slots(nves * ng) * fld);
   if (s) {
     sv->free_dl();
     return s;
@@ -687,16 +712,18 @@ int fork_far(ves3d_sv* sv, int* nseg, cudaEvent_t ev_far0, cudaEvent_t ev_far1, 
   const DevTables& T = sv->tab->d;
   int s;
   cudaStream_t fs = sv->overlap ? sv->side : sv->stream;
-  if (!sv->part) {  // (an order group of a polydisperse suspension never comes here)
-    const long cap = sv->cap_ves * ngrid_(sv->p);
-    if ((s = dalloc(&sv->part, (size_t)far_slots(cap) * 3 * cap))) return s;
-  }
+  const bool f32 = sv->prec == VES3D_PREC_MIXED && !sv->far_force_fp64, dl32 = f32 && sv->far_dl_f32;
+  // (an order group of a polydisperse suspension never comes here)
+  const long cap = sv->cap_ves * ngrid_(sv->p);
+  long sets = 0, sets_dl = 0;
+  if ((s = sv->far_sl.get(f32, sv->npts(), cap, &sv->part, &sets))) return s;
+  if (dl && (s = sv->far_dl.get(dl32, sv->npts(), cap, &sv->part_dl, &sets_dl))) return s;
   VES3D_CK(cudaEventRecord(sv->ev_fork, sv->stream));
   VES3D_CK(cudaStreamWaitEvent(fs, sv->ev_fork, 0));
   if ((s = launch_far_density(sv->F, sv->area, sv->nves, sv->p, T.smooth_w0, sv->den, fs))) return s;
   if (ev_far0) VES3D_CK(cudaEventRecord(ev_far0, fs));
-  if ((s = launch_far(sv->prec == VES3D_PREC_MIXED && !sv->far_force_fp64, sv->pos, sv->den, sv->off, sv->nves,
-                      sv->npts(), ngrid_(sv->p), nullptr, nullptr, nullptr, sv->part, sv->part_slots(), fs, nseg)))
+  if ((s = launch_far(f32, sv->pos, sv->den, sv->off, sv->nves, sv->npts(), ngrid_(sv->p), nullptr, nullptr, nullptr,
+                      sv->part, sets, fs, nseg)))
     return s;
   if (ev_far1) VES3D_CK(cudaEventRecord(ev_far1, fs));
   sv->nseg_dl = 0;
@@ -704,9 +731,8 @@ int fork_far(ves3d_sv* sv, int* nseg, cudaEvent_t ev_far0, cudaEvent_t ev_far1, 
     if ((s = launch_unit_normals(sv->Xt, sv->Xp, sv->nves, sv->p, sv->nrm, fs))) return s;
     if ((s = launch_far_density(sv->G, sv->area, sv->nves, sv->p, T.smooth_w0, sv->dden, fs))) return s;
     if (ev_far0) VES3D_CK(cudaEventRecord(sv->ev[8], fs));
-    const bool dl32 = sv->prec == VES3D_PREC_MIXED && !sv->far_force_fp64 && sv->far_dl_f32;
     if ((s = launch_far_dl(dl32, sv->pos, sv->nrm, sv->dden, sv->off, sv->nves, sv->npts(), ngrid_(sv->p),
-                           sv->part_dl, sv->part_slots(), fs, &sv->nseg_dl)))
+                           sv->part_dl, sets_dl, fs, &sv->nseg_dl)))
       return s;
     if (ev_far0) VES3D_CK(cudaEventRecord(sv->ev[9], fs));
   }
@@ -3153,15 +3179,16 @@ struct ves3d_svp {
   std::vector<long> gnv, gpt0;         // vesicles and first point of each run
   long nves = 0, N = 0;
   int max_nt = 0;
-  double *pos = nullptr, *den = nullptr, *vself = nullptr, *V = nullptr, *Vfar = nullptr, *part = nullptr;
+  double *pos = nullptr, *den = nullptr, *vself = nullptr, *V = nullptr, *Vfar = nullptr;
+  FarPart far_sl, far_dl;  // partial sums of the far field's two layers
   long* off = nullptr;
   long capN = 0, capV = 0;
   bool have_den = false;
   // double layer: a density set by ves3d_svp_set_density_dl (in the groups' G buffers), or
-  // the implicit step's (1 - lambda) u under a viscosity contrast; unit normals, weighted
-  // densities and far partials over all points
+  // the implicit step's (1 - lambda) u under a viscosity contrast; unit normals and weighted
+  // densities over all points
   bool have_dl = false;
-  double *nrm = nullptr, *dden = nullptr, *part_dl = nullptr;
+  double *nrm = nullptr, *dden = nullptr;
   std::vector<double> lam;  // viscosity contrast: one value, or one per vesicle
   bool contrast = false;
   cudaEvent_t ev[4] = {};
@@ -3186,13 +3213,13 @@ struct ves3d_svp {
     graph_exec = nullptr;
     graph = nullptr;
   }
-  // sets of far-field partial sums of the current points that the buffers (sized for capN) hold
-  long part_slots() const { return far_slots(capN) * capN / N; }
   void free_global() {
-    double* ps[] = {pos, den, vself, V, Vfar, part, nrm, dden, part_dl};
+    double* ps[] = {pos, den, vself, V, Vfar, nrm, dden};
     for (double* q : ps) dfree(q);
+    far_sl.free();
+    far_dl.free();
     dfree(off);
-    pos = den = vself = V = Vfar = part = nrm = dden = part_dl = nullptr;
+    pos = den = vself = V = Vfar = nrm = dden = nullptr;
     off = nullptr;
     capN = capV = 0;
   }
@@ -3303,7 +3330,6 @@ int ves3d_svp_set_src_coord(ves3d_svp* g, const double* S, const int* orders, lo
     s |= dalloc(&g->vself, 3 * (size_t)pt);
     s |= dalloc(&g->V, 3 * (size_t)pt);
     s |= dalloc(&g->Vfar, 3 * (size_t)pt);
-    s |= dalloc(&g->part, (size_t)far_slots(pt) * 3 * pt);
     s |= dalloc(&g->off, (size_t)n_ves + 1);
     if (s) {
       g->free_global();
@@ -3336,7 +3362,7 @@ int ves3d_svp_set_density_sl(ves3d_svp* g, const double* f, int is_device) {
   return VES3D_OK;
 }
 
-// Double-layer buffers of the suspension (normals, weighted densities, far partials) and of
+// Double-layer buffers of the suspension (normals, weighted densities) and of
 // every group (density, coefficients, self matrices).
 static int svp_alloc_dl(ves3d_svp* g) {
   int s = 0;
@@ -3345,12 +3371,10 @@ static int svp_alloc_dl(ves3d_svp* g) {
   if (g->nrm) return VES3D_OK;
   s |= dalloc(&g->nrm, 3 * (size_t)g->capN);
   s |= dalloc(&g->dden, 3 * (size_t)g->capN);
-  s |= dalloc(&g->part_dl, (size_t)far_slots(g->capN) * 3 * g->capN);
   if (s) {
     dfree(g->nrm);
     dfree(g->dden);
-    dfree(g->part_dl);
-    g->nrm = g->dden = g->part_dl = nullptr;
+    g->nrm = g->dden = nullptr;
   }
   return s;
 }
@@ -3423,6 +3447,11 @@ static int svp_self_parts(ves3d_svp* g, bool dl) {
 static int svp_far(ves3d_svp* g, bool dl) {
   NvtxRange nvtx("ves3d far");
   const bool mixed = g->prec == VES3D_PREC_MIXED && !g->far_force_fp64;
+  double *part = nullptr, *part_dl = nullptr;
+  long sets = 0, sets_dl = 0;
+  int s, nseg = 0, nseg_dl = 0;
+  if ((s = g->far_sl.get(mixed, g->N, g->capN, &part, &sets))) return s;
+  if (dl && (s = g->far_dl.get(mixed && g->far_dl_f32, g->N, g->capN, &part_dl, &sets_dl))) return s;
   std::vector<FarGroup> fg;
   long v0 = 0;
   for (size_t r = 0; r < g->grp.size(); r++) {
@@ -3431,16 +3460,15 @@ static int svp_far(ves3d_svp* g, bool dl) {
   }
   if (!dl)
     return launch_far_groups(mixed, g->pos, g->den, g->off, g->nves, g->N, fg.data(), (int)fg.size(), g->vself, g->V,
-                             g->Vfar, g->part, g->part_slots(), g->stream);
-  int s, nseg = 0, nseg_dl = 0;
+                             g->Vfar, part, sets, g->stream);
   if ((s = launch_far_groups(mixed, g->pos, g->den, g->off, g->nves, g->N, fg.data(), (int)fg.size(), nullptr,
-                             nullptr, nullptr, g->part, g->part_slots(), g->stream, &nseg)))
+                             nullptr, nullptr, part, sets, g->stream, &nseg)))
     return s;
   if ((s = launch_far_dl_groups(mixed && g->far_dl_f32, g->pos, g->nrm, g->dden, g->off, g->nves, g->N, fg.data(),
-                                (int)fg.size(), g->part_dl, g->part_slots(), g->stream, &nseg_dl)))
+                                (int)fg.size(), part_dl, sets_dl, g->stream, &nseg_dl)))
     return s;
-  return launch_far_reduce(g->part, nseg, g->off, g->nves, g->N, g->vself, g->V, g->Vfar, g->stream, g->part_dl,
-                           nseg_dl, kDl);
+  return launch_far_reduce(part, nseg, g->off, g->nves, g->N, g->vself, g->V, g->Vfar, g->stream, part_dl, nseg_dl,
+                           kDl);
 }
 
 int ves3d_svp_capture_eval(ves3d_svp* g) {
