@@ -74,7 +74,43 @@ struct TablesOwner {
                     d.syn1_leg_t, d.syn1_dleg_t, d.ring_leg, d.ring_dleg, d.ring_twiddle, d.ring_off};
     for (void* p : ptrs) dfree(p);
   }
-  int upload(cudaStream_t st) {
+  // The fused FP64 build's tables, once (a context whose builds run on the tensor cores has no use for
+  // them until it takes an implicit step or a double layer).
+  int upload_ring(cudaStream_t st) {
+    const size_t nc = (size_t)ncoef_(h.p0), nl = (size_t)h.p1 + 1;
+    if (d.ring_off || !ring_supported(h.p0, h.p1)) return VES3D_OK;
+    const std::vector<int> lo = ring_leg_offsets(h.p0);
+    const size_t ldl = lo.back();
+    const double scale = std::sqrt(2.0 * M_PI);
+    std::vector<double> ra(ldl * nl, 0.0), rb(ldl * nl, 0.0);
+    for (size_t l = 0; l < nl; l++)
+      for (int k = 0; k < 2 * h.p0; k++) {
+        const int b0 = h.blk_off[k], len = h.blk_off[k + 1] - b0;
+        for (int i = 0; i < len; i++) {  // even degrees of the block first
+          const size_t o = l * ldl + lo[2 * k + i % 2] + i / 2;
+          ra[o] = h.syn1.leg[(b0 + i) * nl + l] * scale;
+          rb[o] = h.syn1.dleg[(b0 + i) * nl + l] * scale;
+        }
+      }
+    const int pad = ring_padded_order(h.p0, h.p1);
+    std::vector<double> tw;
+    for (int j = 0; pad && j <= h.p1 / 2; j++)
+      for (int m = 0; m <= pad; m++) {
+        const double a = M_PI * ((long)m * j % (2 * h.p1)) / h.p1;
+        tw.push_back(std::cos(a));
+        tw.push_back(std::sin(a));
+      }
+    d.ring_ldl = (int)ldl;
+    for (double** t : {&d.ring_leg, &d.ring_dleg, &d.ring_twiddle}) {  // (of an attempt that failed)
+      dfree(*t);
+      *t = nullptr;
+    }
+    int s = dupload(&d.ring_leg, ra, st);
+    if (!s) s = dupload(&d.ring_dleg, rb, st);
+    if (!s) s = dupload(&d.ring_twiddle, tw, st);
+    return s ? s : dupload(&d.ring_off, lo, st);
+  }
+  int upload(cudaStream_t st, bool ring = false) {
     d.p0 = h.p0;
     d.p1 = h.p1;
     d.mr_total = (int)h.mr.size();
@@ -99,34 +135,8 @@ struct TablesOwner {
           }
         s |= dupload(&d.syn1_leg_t, a, st);
         s |= dupload(&d.syn1_dleg_t, b, st);
-        const std::vector<int> lo = ring_leg_offsets(h.p0);
-        const size_t ldl = lo.back();
-        const double scale = std::sqrt(2.0 * M_PI);
-        std::vector<double> ra(ldl * nl, 0.0), rb(ldl * nl, 0.0);
-        for (size_t l = 0; l < nl; l++)
-          for (int k = 0; k < 2 * h.p0; k++) {
-            const int b0 = h.blk_off[k], len = h.blk_off[k + 1] - b0;
-            for (int i = 0; i < len; i++) {  // even degrees of the block first
-              const size_t o = l * ldl + lo[2 * k + i % 2] + i / 2;
-              ra[o] = a[l * nc + b0 + i] * scale;
-              rb[o] = b[l * nc + b0 + i] * scale;
-            }
-          }
-        d.ring_ldl = (int)ldl;
-        s |= dupload(&d.ring_off, lo, st);
-        s |= dupload(&d.ring_leg, ra, st);
-        s |= dupload(&d.ring_dleg, rb, st);
       }
     }
-    const int pad = ring_supported(h.p0, h.p1) ? ring_padded_order(h.p0, h.p1) : 0;
-    std::vector<double> tw;
-    for (int j = 0; pad && j <= h.p1 / 2; j++)
-      for (int m = 0; m <= pad; m++) {
-        const double a = M_PI * ((long)m * j % (2 * h.p1)) / h.p1;
-        tw.push_back(std::cos(a));
-        tw.push_back(std::sin(a));
-      }
-    s |= dupload(&d.ring_twiddle, tw, st);
     s |= dupload(&d.syn1_four, h.syn1.four, st);
     s |= dupload(&d.syn1_dfour, h.syn1.dfour, st);
     s |= dupload(&d.synT_four, h.synT.four, st);
@@ -148,6 +158,7 @@ struct TablesOwner {
     s |= dupload(&d.sin_tab, h.sin_tab, st);
     s |= dupload(&d.syn0_d2leg, h.syn0_d2leg, st);
     s |= dupload(&d.syn0_d2four, h.syn0_d2four, st);
+    if (ring) s |= upload_ring(st);
     if (s) return VES3D_ERR_NOMEM;
     VES3D_CK(cudaStreamSynchronize(st));
     return VES3D_OK;
@@ -611,6 +622,7 @@ int run_setup(ves3d_sv* sv, bool dl, bool wait) {
     set_error("internal: self-matrix build without its buffers");
     return VES3D_ERR_STATE;
   }
+  if (fused && !tc && (s = sv->tab->upload_ring(st))) return s;
   if (tc && !sv->tc_err) {
     if ((s = dalloc(&sv->tc_err, 1))) return s;
     VES3D_CK(cudaMemsetAsync(sv->tc_err, 0, sizeof(int), st));
@@ -988,7 +1000,7 @@ int ves3d_sv_create(int sh_order, int sh_order_up, int precision, int device, ve
   VES3D_CK(cudaEventCreateWithFlags(&sv->ev_src, cudaEventDisableTiming));
   sv->tab.reset(new TablesOwner());
   build_tables(sh_order, sh_order_up, sv->tab->h);
-  int s = sv->tab->upload(sv->stream);
+  int s = sv->tab->upload(sv->stream, /*ring=*/!(precision == VES3D_PREC_MIXED && tc_build_supported(sh_order, sh_order_up)));
   if (s) return s;
   *out = sv.release();
   return VES3D_OK;
@@ -1196,7 +1208,8 @@ int ves3d_sv_set_order_up(ves3d_sv* sv, int sh_order_up) {
   if (sh_order_up == sv->pup) return VES3D_OK;
   std::unique_ptr<TablesOwner> t(new TablesOwner());
   build_tables(sv->p, sh_order_up, t->h);
-  if ((s = t->upload(sv->stream))) return s;
+  if ((s = t->upload(sv->stream, /*ring=*/!(sv->prec == VES3D_PREC_MIXED && tc_build_supported(sv->p, sh_order_up)))))
+    return s;
   VES3D_CK(cudaDeviceSynchronize());  // nothing queued still reads the old tables
   sv->tab = std::move(t);
   sv->pup = sh_order_up;
