@@ -1728,6 +1728,19 @@ struct InteractionWorkspace {
   double* buf = nullptr;  // sources, densities, potentials, then the partial sums of the paired form
   size_t cap = 0;
   cudaStream_t st = nullptr;
+  bool grow(size_t need) {
+    if (cap >= need) return true;
+    if (buf) cudaFree(buf);
+    buf = nullptr;
+    cap = 0;
+    if (cudaMalloc((void**)&buf, need * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();  // reported here, not by the next launch
+      buf = nullptr;
+      return false;
+    }
+    cap = need;
+    return true;
+  }
 };
 
 void ves3d_stokes_alltoall_f64(const double* src, const double* den, size_t np, double* pot, void** ctx) {
@@ -1746,18 +1759,13 @@ void ves3d_stokes_alltoall_f64(const double* src, const double* den, size_t np, 
     if (!*ctx) *ctx = new InteractionWorkspace();
     ws = (InteractionWorkspace*)*ctx;
   }
-  const long slots = alltoall_slots((long)np);
-  const size_t need = (9 + 3 * (size_t)slots) * np;
-  if (ws->cap < need) {
-    if (ws->buf) cudaFree(ws->buf);
-    ws->buf = nullptr;
-    ws->cap = 0;
-    if (cudaMalloc((void**)&ws->buf, need * sizeof(double)) != cudaSuccess) {
-      set_error("cudaMalloc of %zu bytes failed", need * sizeof(double));
-      fail();
-      return;
-    }
-    ws->cap = need;
+  // partial sums of up to a GiB; without room for them the one-sided sums, which need none
+  long slots = alltoall_slots((long)np);
+  if (slots && !ws->grow((9 + 3 * (size_t)slots) * np)) slots = 0;
+  if (!slots && !ws->grow(9 * np)) {
+    set_error("cudaMalloc of %zu bytes failed", 9 * np * sizeof(double));
+    fail();
+    return;
   }
   if (!ws->st && cudaStreamCreateWithFlags(&ws->st, cudaStreamNonBlocking) != cudaSuccess) {
     set_error("cudaStreamCreate failed");
