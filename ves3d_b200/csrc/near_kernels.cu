@@ -34,7 +34,7 @@ namespace {
 
 constexpr int kInterpDeg = 8;
 constexpr double kSqrt2Pi = 2.5066282746310002;
-constexpr double kStepDone = 1e-14;  // a Gauss-Newton step (radians) of no effect on the values
+constexpr double kStepDone = 1e-15;  // a Gauss-Newton step (radians) below the rounding of the angles
 
 __device__ __forceinline__ double inter_point(int i) { return i ? 1.0 + (i - 1.0) / (kInterpDeg - 2) : 0.0; }
 
@@ -276,7 +276,7 @@ constexpr int kProjWarps = 4;
 // use are neighbours). The vesicle's coefficients and the recurrence tables are staged in shared
 // memory. What bounds it is the serial chain of up to 40 Gauss-Newton steps of p + 1 recurrence
 // steps each: with the square roots and divisions of the recurrence in tables, 16 lanes per pair
-// at p <= 15 and every warp at it, 15,000 pairs at p = 12 take 0.89 ms (one warp of a 128-thread CTA
+// at p <= 15 and every warp at it, 15,000 pairs at p = 12 take 0.98 ms (one warp of a 128-thread CTA
 // per pair, three waiting, and the coefficients recomputed took 14.5 ms with the sums of
 // k_near_correct).
 template <int G>
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(32 * kProjWarps) k_near_project(NearArgs A) {
       th += d1;
       ph += d2;
     }
-    // at this length the steps are the rounding of the surface itself
+    // at this length the steps are the rounding of the angles
     done = done || fmax(fabs(d1), fabs(d2)) < kStepDone;
   }
   sh_point<G>(Sg, tab, p, bo, cos(th), ph, true, val);
