@@ -114,4 +114,14 @@ __device__ __forceinline__ double rsqrt_f64(double r2) {
   return fma(y * e, c, y);
 }
 
+// num / s from si = 1.0 / s: a first quotient, its remainder by one fused multiply-add and one correction
+// (Markstein, IBM J. Res. Dev. 34, 1990). The first quotient may be up to 1.5 units off, beyond that
+// paper's theorem, so that the result's last bit rests on the comparison with the division (none of
+// 2.7e8 quotients on the device differs). For s in [2^-27, 1] and num zero (its sign is lost) or
+// |num| > 2^-900; a lane that shares si among many numerators saves their divisions.
+__device__ __forceinline__ double quotient_by(double num, double s, double si) {
+  const double q = num * si;
+  return fma(fma(-q, s, num), si, q);
+}
+
 }  // namespace ves3d

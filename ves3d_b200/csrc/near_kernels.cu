@@ -210,11 +210,9 @@ __device__ __forceinline__ void sh_point(const double* __restrict__ S, const dou
     const double pnext = __shfl_down_sync(0xffffffffu, pn, 1, G);
     if (act && n >= m) {
       const double c2 = row[64];
-      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta); the quotient by s from its reciprocal, one
-      // remainder and one correction (Markstein, IBM J. Res. Dev. 34, 1990), which round correctly
+      // -(legpoly_deriv) = d/dtheta of P(m, n)(cos theta)
       const double num = m * x * pn + c2 * s * (m + 1 <= n ? pnext : 0.0);
-      const double q0 = num * si;
-      const double dpn = s > 0.0 ? fma(fma(-q0, s, num), si, q0) : 0.0;
+      const double dpn = s > 0.0 ? quotient_by(num, s, si) : 0.0;
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const double a = Sc[d * nc + n];
