@@ -159,7 +159,8 @@ int ves3d_sv_launch_eval_graph(ves3d_sv* sv);
  * 256 only, for its accuracy) -- is timed once with CUDA events beside the default shape
  * and the fastest of them all is kept.
  * FP64 sums over 8000 and more points have one form that needs no tuning (every unordered
- * pair evaluated once) unless a shape is fixed. Never tunes during stream capture. */
+ * pair evaluated once, on up to 80 sets of partial sums of 24 bytes a point within a GiB)
+ * unless a shape is fixed. Never tunes during stream capture. */
 int ves3d_set_autotune(int on);
 /* Fix the far-field launch shape instead (waves in {4, 8, 16}, threads per CTA in
  * {256, 384}, targets per thread 2); waves = 0 returns to the default / autotuned shape. */
@@ -492,8 +493,10 @@ int ves3d_cuda_stokes_f32(int src_m, int trg_m, int n, int t_head, int t_tail, c
 /* All-pairs interaction with the reference's VesInteraction handle signature
  * (include/VesInteraction.h:21, matched by StokesAlltoAll, include/CPUKernels.h:46-49):
  * HOST pointers, point-major xyz, np points; pot[t] = sum over all s of the Stokeslet
- * of den[s] (coincident points contribute nothing). *ctx may hold a library-owned
- * workspace between calls; free it with ves3d_interaction_free(ctx). Errors are
+ * of den[s] (coincident points contribute nothing; points nearer than 2^-63 count as such).
+ * *ctx may hold a library-owned workspace between calls (9 values a point, and from 4,000
+ * points on partial sums of up to a GiB where the device has room for them); free it with
+ * ves3d_interaction_free(ctx). Errors are
  * reported through ves3d_last_error() and leave pot filled with NaN. */
 void ves3d_stokes_alltoall_f64(const double* src, const double* den, size_t np, double* pot, void** ctx);
 void ves3d_interaction_free(void** ctx);

@@ -738,7 +738,7 @@ __global__ void k_far_reduce(const double* __restrict__ part, int nseg, const lo
   }
 }
 
-// 128-thread CTAs per vesicle: one round at p = 16 (1632 values). The kernel reads the partial sums
+// 128-thread CTAs per vesicle: 1536 values a round, of 1632 at p = 16. The kernel reads the partial sums
 // once; one CTA per vesicle left 64 vesicles on 64 SMs (69 us, now 26).
 constexpr int kReduceParts = 12;
 

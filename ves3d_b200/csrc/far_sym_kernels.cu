@@ -11,6 +11,9 @@
 //   single layer, 278,528 points 123.2 -> 98.9 ms, 34,816 points 2.20 -> 1.59 ms
 //   double layer, 26,112 points  1.36 -> 1.17 ms
 //   all pairs of 19,000 points   2.14 -> 0.53 ms (one target per thread before)
+// The partial sums are the price: G sets of 24 bytes a point (up to 80, within a GiB; 78 sets, 521 MB, at
+// 278,528 points), where a group of several target blocks reads and adds to what it has written: 734 MB
+// of DRAM traffic a launch against 105 one-sided, of the 640 GB that the launch's time would move.
 // Other shapes (2 to 6 targets, 2 to 16 warps, 80 to 255 registers) ran 97 to 139 ms at 278,528
 // points; two sources a step with sums in shuffles 106 ms.
 #include <algorithm>

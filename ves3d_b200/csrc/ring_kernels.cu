@@ -18,7 +18,7 @@
 // instruction has no use for (FP64 DMMA runs at the vector units' rate); one thread then holds a row's
 // coefficients in registers and meets compile-time cosines as constant operands. A CTA takes one
 // rotation, LPG latitude pairs through all phases at a time.
-// Bound by the FP64 pipe (37% busy at p = 16) and, where it is not, by the barriers between the
+// Bound by the FP64 pipe (39% busy at p = 16) and, where it is not, by the barriers between the
 // phases and instruction fetch of the unrolled transforms. Self matrices of
 //   512 / 64 vesicles, p = 16:  32.8 -> 18.3 ms / 4.12 -> 2.28 ms  (before: dense, DMMA from shared memory)
 //   64 vesicles, p = 24:        32.4 -> 16.3 ms
